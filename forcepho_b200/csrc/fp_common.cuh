@@ -88,6 +88,14 @@ __device__ __forceinline__ float4 fp_ldg_policy(const float4 *p, uint64_t pol)
     return r;
 }
 
+// Two FP32 values for the packed FP32 instructions: one issue slot for two
+// operations, each rounded as its scalar form (the FP32 rate is the same).
+typedef float2 fp_f2;
+struct __align__(16) fp_f4 {
+    fp_f2 x, y;
+};
+__device__ __forceinline__ fp_f2 fp_dup(float x) { return make_float2(x, x); }
+
 // 2x2 matrices as {m11, m12, m21, m22}
 template <typename R>
 struct fp_m22 {

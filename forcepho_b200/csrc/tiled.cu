@@ -23,15 +23,18 @@
 //                     the hits; y terms once per row of pixels; SFU ex2; FP32
 //                     runs flushed into per-pixel FP64 sums; residual, chi2
 //                     term in f64, w = r ierr^2;
-//                  3. adjoint, Gaussian-parallel: one Gaussian per lane, the
-//                     tile's nonzero-weight pixels broadcast from shared memory
-//                     (a chunk's last, partial group of v Gaussians is
-//                     replicated over the idle lanes, each replica taking every
-//                     k-th pixel, and the replicas summed by shuffles);
-//                     each lane accumulates 12 moments (FP32 runs -> FP64) from
-//                     which the 6 image-space partials follow exactly; the FP64
-//                     Jacobian maps them to the 7 on-sky partials once per
-//                     (Gaussian, segment), not once per pixel;
+//                  3. adjoint, Gaussian-parallel: one Gaussian per lane.  The
+//                     tile's weights lie in shared memory as a dense grid of
+//                     its cell, walked down strips of 4 columns, or, where
+//                     the pixels do not fill such a grid, as a list of
+//                     nonzero-weight pixels that is broadcast to the lanes (a
+//                     chunk's last, partial group of v Gaussians is
+//                     replicated over the idle lanes, each replica taking
+//                     every k-th row or pixel, and the replicas summed by
+//                     shuffles).  Power sums of the offsets give the 6
+//                     image-space partials, which the FP64 Jacobian maps to
+//                     the 7 on-sky partials once per (Gaussian, segment), not
+//                     once per pixel;
 //                  4. per-source sums inside each warp (a segmented shuffle
 //                     tree), one fixed-order sum over the warps per tile ->
 //                     per-tile partials.
@@ -240,11 +243,41 @@ __device__ __forceinline__ float2 tile_origin(const fp_tile &tl)
     return make_float2(isfinite(ox) ? ox : 0.f, isfinite(oy) ? oy : 0.f);
 }
 
+// A tile's dense weight grid (grid_partials): its size, the relative
+// coordinates of its first place, and per strip of 4 columns the rows
+// [lo, lo + n) with weighted pixels, packed as 64 lo + n.
+struct tile_grid {
+    bool on;
+    int cols, rows;
+    float x0, y0;
+    int strip[8];
+};
+constexpr int FP_GRID_STRIDE = 36;      // floats per row: 8 replicas' rows start in different banks
+
+// Whether a tile's box allows the grid: its pixels lie within the cell of its
+// class, which the planner's compact tiles do, and the box starts at integers.
+__device__ __forceinline__ tile_grid tile_grid_of(const fp_tile &tl, const float ox, const float oy, bool allowed)
+{
+    tile_grid g;
+    g.cols = tl.tile_pixels == 256 ? 16 : 32;
+    g.rows = tl.tile_pixels == 1024 ? 32 : 16;
+    g.x0 = tl.bbox[0] - ox;
+    g.y0 = tl.bbox[2] - oy;
+    g.on = allowed && tl.bbox[1] - tl.bbox[0] < (float)g.cols && tl.bbox[3] - tl.bbox[2] < (float)g.rows &&
+           g.x0 == truncf(g.x0) && g.y0 == truncf(g.y0);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) g.strip[j] = 0;
+    return g;
+}
+
 // Forward pass of one tile, P pixels per thread (the tile holds at most
 // 256 P pixels): the model of each pixel over the tile's kept Gaussians, the
 // residual (written out when the patch has a residual array), the chi2 terms
 // reduced into s_red[FP_WARPS], and the nonzero-weight pixels (x, y, w) compacted
 // into s_pix in ascending order.  Returns their count (the same on every thread).
+// With s_rows, the weights go into the dense grid of grid_partials at s_pix
+// instead, if every weighted pixel has a place of its own there (grid.on is
+// then left true); x0, y0 are the relative coordinates of its first place.
 // Pixel coordinates and Gaussian centres are taken relative to the tile's
 // origin (ox, oy) (stage_gauss); the boxes stay absolute.
 template <int P>
@@ -253,10 +286,17 @@ __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure
                                             const float4 *__restrict__ gfwd, const float4 *__restrict__ gbox,
                                             const float2 *__restrict__ gctr, const float ox, const float oy,
                                             const bool nocull, const int gc, const uint16_t *s_idx, float4 *s_ga,
-                                            float4 *s_gb, float4 *s_gbox, float4 *s_pix, int *s_int, double *s_red)
+                                            float4 *s_gb, float4 *s_gbox, float4 *s_pix, int *s_int, double *s_red,
+                                            unsigned *s_rows, tile_grid &grid)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int npix = tl.n_pix;
+    if (grid.on) {
+        // the previous tile's readers are past their last barrier
+        for (int i = tid; i < grid.rows * FP_GRID_STRIDE / 4; i += FP_THREADS)
+            s_pix[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (tid < 32) s_rows[tid] = 0u;
+    }
 
     // the tile's pixels are listed in the plan's pixel order (compact cells)
     const int j0 = tid * P;
@@ -447,7 +487,20 @@ __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure
     for (int o = 16; o > 0; o >>= 1) chi += __shfl_down_sync(0xffffffffu, chi, o);
     if (lane == 31) s_int[8 + warp] = incl;
     if (lane == 0) s_red[warp] = chi;
-    __syncthreads();
+    bool fits = grid.on;
+    if (grid.on) {
+        if (gc == 0) __syncthreads();       // no pass over Gaussians ordered the clearing above
+#pragma unroll
+        for (int k = 0; k < P; ++k)
+            if (ws[k] != 0.f) {
+                const float gx = xs[k] - grid.x0, gy = ys[k] - grid.y0;
+                const bool in = isfinite(ws[k]) && gx >= 0.f && gx < (float)grid.cols && gy >= 0.f &&
+                                gy < (float)grid.rows && gx == truncf(gx) && gy == truncf(gy);
+                fits = fits && in;
+                if (in) atomicOr(&s_rows[(int)gy], 1u << (int)gx);
+            }
+    }
+    grid.on = __syncthreads_and(fits ? 1 : 0) != 0;
     int off = incl - nz, nzt = 0;
 #pragma unroll
     for (int w = 0; w < FP_WARPS; ++w) {
@@ -455,9 +508,41 @@ __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure
         off += (w < warp) ? cnt : 0;
         nzt += cnt;
     }
+    if (grid.on) {
+        // as many places as pixels: no two share one; and at least half of the
+        // strips' places in use, else the list does less work
+        const unsigned row = s_rows[lane];
+        int places = __popc(row), span = 0;
 #pragma unroll
-    for (int k = 0; k < P; ++k)
-        if (ws[k] != 0.f) s_pix[off++] = make_float4(xs[k], ys[k], ws[k], 0.f);
+        for (int o = 16; o > 0; o >>= 1) places += __shfl_xor_sync(0xffffffffu, places, o);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const unsigned b = __ballot_sync(0xffffffffu, (row >> (4 * j)) & 0xfu);
+            if (b) {
+                const int lo = __ffs(b) - 1, n = 32 - __clz(b) - lo;
+                grid.strip[j] = 64 * lo + n;
+                span += 4 * n;
+            }
+        }
+        grid.on = places == nzt && span <= 2 * nzt;
+    }
+    if (grid.on) {
+        float *s_w = reinterpret_cast<float *>(s_pix);
+        if (tid == 0) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s_int[16 + j] = grid.strip[j];
+        }
+#pragma unroll
+        for (int k = 0; k < P; ++k)
+            if (ws[k] != 0.f) {
+                const int gx = (int)(xs[k] - grid.x0), gy = (int)(ys[k] - grid.y0);
+                s_w[gy * FP_GRID_STRIDE + gx] = ws[k];
+            }
+    } else {
+#pragma unroll
+        for (int k = 0; k < P; ++k)
+            if (ws[k] != 0.f) s_pix[off++] = make_float4(xs[k], ys[k], ws[k], 0.f);
+    }
     if (tid == 0) {
         double t = 0.0;
 #pragma unroll
@@ -562,20 +647,28 @@ __device__ __forceinline__ void adjoint_moments(const float4 A, const float4 B,
 }
 #endif
 
-// Image-space partials from the moments (the reference's dC/d{A,x,y,Fxx,Fyy,Fxy}
-// summed over pixels, common_kernel.cc:118-132), then the Jacobian to the 7
-// on-sky partials (common_kernel.cc:135-141), all in FP64.
-__device__ __forceinline__ void moments_to_grad(const double *__restrict__ J, const double (&m)[12],
-                                                double (&g)[NPARAMS])
+// Image-space partials S = dC/d{A, x, y, Fxx, Fyy, Fxy} summed over pixels
+// (common_kernel.cc:118-132), all but the first without their factor amp, from
+// the moments of the pixel list, in FP64.
+__device__ __forceinline__ void moments_to_partials(const double *__restrict__ J, const double (&m)[12],
+                                                    double (&S)[6])
 {
-    const double amp = J[0], fxx = J[1], fxy = J[2], fyy = J[3];
+    const double fxx = J[1], fxy = J[2], fyy = J[3];
     const double ic = 1.0 / FP_EXP2_SCALE;
-    const double SA = m[1];
-    const double Sx = amp * ic * (m[2] - (fxx * m[4] + fxy * m[5]) * (1.0 / 12.0));
-    const double Sy = amp * ic * (m[3] - (fyy * m[5] + fxy * m[4]) * (1.0 / 12.0));
-    const double Sfx = amp * (-0.5 * m[6] - m[0] * (1.0 / 24.0) + ic * m[9] * (1.0 / 12.0));
-    const double Sfy = amp * (-0.5 * m[7] - m[0] * (1.0 / 24.0) + ic * m[10] * (1.0 / 12.0));
-    const double Sfxy = amp * (-m[8] + ic * m[11] * (1.0 / 12.0));
+    S[0] = m[1];
+    S[1] = ic * (m[2] - (fxx * m[4] + fxy * m[5]) * (1.0 / 12.0));
+    S[2] = ic * (m[3] - (fyy * m[5] + fxy * m[4]) * (1.0 / 12.0));
+    S[3] = -0.5 * m[6] - m[0] * (1.0 / 24.0) + ic * m[9] * (1.0 / 12.0);
+    S[4] = -0.5 * m[7] - m[0] * (1.0 / 24.0) + ic * m[10] * (1.0 / 12.0);
+    S[5] = -m[8] + ic * m[11] * (1.0 / 12.0);
+}
+
+// The Jacobian to the 7 on-sky partials (common_kernel.cc:135-141), in FP64.
+__device__ __forceinline__ void partials_to_grad(const double *__restrict__ J, const double (&S)[6],
+                                                 double (&g)[NPARAMS])
+{
+    const double amp = J[0], SA = S[0];
+    const double Sx = amp * S[1], Sy = amp * S[2], Sfx = amp * S[3], Sfy = amp * S[4], Sfxy = amp * S[5];
     g[0] = J[4] * SA;
     g[1] = J[5] * Sx + J[6] * Sy;
     g[2] = J[7] * Sx + J[8] * Sy;
@@ -584,6 +677,107 @@ __device__ __forceinline__ void moments_to_grad(const double *__restrict__ J, co
     g[5] = J[17] * SA;
     g[6] = J[18] * SA;
 }
+
+#ifndef FP_KAHAN
+// ---------------------------------------------------------------------------
+// adjoint over a pixel grid
+// ---------------------------------------------------------------------------
+// A tile whose weighted pixels sit on distinct integer positions of its cell
+// (32x32, 32x16 or 16x16) keeps their weights in a dense grid instead of a
+// list, FP_GRID_STRIDE floats per row.  One lane walks its Gaussian down the
+// rows r, r + step, ... < rend of one strip of 4 columns: s_w is the strip's
+// first column, x its coordinate, y0 that of row 0.
+//
+// FP32 operations bound the adjoint.  The list takes 30 per pixel: the
+// offsets, the exponent, H and 12 sums, all about the Gaussian's own centre.
+// Here
+//   * H is a quadratic form of the offsets, so every moment of K and KH is a
+//     combination of the 15 sums of K dx^i dy^j, i + j <= 4;
+//   * down a column dx is fixed: 5 sums of K dy^j per column, weighted with
+//     dx^i once at the strip's end, stand for all 15;
+//   * the exponent is dx^2 Fxx + dy (2 Fxy dx + Fyy dy), two operations with
+//     the column's products formed beforehand.
+// That leaves 9 operations per pixel, paired over columns (packed FP32), and
+// 2 per row of 4 pixels.  Four columns are what 64 registers hold (10 sums
+// each pair).  Sums run over at most 32 rows in FP32, as the list's do; the
+// step from the 15 sums to the image-space partials is FP64.  Sums about the
+// strip's centre instead, with constant weights, ran 5 % faster but cost
+// Gaussians narrower than the strip two decimal digits when shifted.
+// Tile kernel on 48 field patches (2.9e9 evaluated pairs): 6.31 ms with the
+// list, 4.02 ms here; on a 30-source patch of 32 exposures of 256x256 px,
+// 1.64 and 0.98 ms.
+__device__ __forceinline__ void grid_partials(const float4 A, const float4 B, const double *__restrict__ J,
+                                              const float *__restrict__ s_w, int r, int rend, int step, float x,
+                                              float y0, double (&S)[6])
+{
+    float dx[4], m[5][5];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) dx[k] = (x + (float)k) - A.x;
+    {
+        const fp_f2 nyc = fp_dup(-A.y), fyy = fp_dup(B.x), ystep = fp_dup((float)step);
+        fp_f2 y = fp_dup(y0 + (float)r);
+        fp_f2 l[2], q[2], Y[5][2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            l[k] = make_float2((2.f * A.w) * dx[2 * k], (2.f * A.w) * dx[2 * k + 1]);
+            q[k] = make_float2((A.z * dx[2 * k]) * dx[2 * k], (A.z * dx[2 * k + 1]) * dx[2 * k + 1]);
+#pragma unroll
+            for (int j = 0; j < 5; ++j) Y[j][k] = fp_dup(0.f);
+        }
+        const float *pw = s_w + r * FP_GRID_STRIDE;
+        const float *pend = s_w + rend * FP_GRID_STRIDE;
+#pragma unroll 1
+        for (; pw < pend; pw += step * FP_GRID_STRIDE) {
+            const fp_f4 w = *reinterpret_cast<const fp_f4 *>(pw);
+            const fp_f2 dy = __fadd2_rn(y, nyc);
+            y = __fadd2_rn(y, ystep);
+            const fp_f2 yy = __fmul2_rn(dy, dy);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const fp_f2 e = __ffma2_rn(dy, __ffma2_rn(fyy, dy, l[k]), q[k]);
+                const fp_f2 g = __fmul2_rn(k ? w.y : w.x, make_float2(fp_ex2(e.x), fp_ex2(e.y)));
+                const fp_f2 K = make_float2((e.x < FP_CUT_SCALED) ? 0.f : g.x, (e.y < FP_CUT_SCALED) ? 0.f : g.y);
+                Y[0][k] = __fadd2_rn(Y[0][k], K);
+                Y[1][k] = __ffma2_rn(K, dy, Y[1][k]);
+                const fp_f2 t = __fmul2_rn(K, yy);
+                Y[2][k] = __fadd2_rn(Y[2][k], t);
+                Y[3][k] = __ffma2_rn(t, dy, Y[3][k]);
+                Y[4][k] = __ffma2_rn(t, yy, Y[4][k]);
+            }
+        }
+        // m[i][j] = sum K dx^i dy^j over the strip
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+            const float t[4] = {Y[j][0].x, Y[j][0].y, Y[j][1].x, Y[j][1].y};
+            m[0][j] = (t[0] + t[1]) + (t[2] + t[3]);
+            float p[4] = {t[0], t[1], t[2], t[3]};
+#pragma unroll
+            for (int i = 1; i < 5 - j; ++i) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) p[k] *= dx[k];
+                m[i][j] = (p[0] + p[1]) + (p[2] + p[3]);
+            }
+        }
+    }
+    // H = h + |F dx|^2 / 24, h = 1 - tr F / 24
+    const double a = J[1], b = J[2], c = J[3];
+    const double t = a + c;
+    const double xx = a * a + b * b, xy = b * t, yy = b * b + c * c;      // F^2
+    const double h = 1.0 - t * (1.0 / 24.0);
+    const double p = xx * (1.0 / 24.0), q = xy * (1.0 / 12.0), s = yy * (1.0 / 24.0);
+    const double H10 = h * m[1][0] + p * m[3][0] + q * m[2][1] + s * m[1][2];
+    const double H01 = h * m[0][1] + p * m[2][1] + q * m[1][2] + s * m[0][3];
+    const double H20 = h * m[2][0] + p * m[4][0] + q * m[3][1] + s * m[2][2];
+    const double H11 = h * m[1][1] + p * m[3][1] + q * m[2][2] + s * m[1][3];
+    const double H02 = h * m[0][2] + p * m[2][2] + q * m[1][3] + s * m[0][4];
+    S[0] += h * m[0][0] + p * m[2][0] + q * m[1][1] + s * m[0][2];
+    S[1] += a * H10 + b * H01 - (xx * m[1][0] + xy * m[0][1]) * (1.0 / 12.0);
+    S[2] += b * H10 + c * H01 - (xy * m[1][0] + yy * m[0][1]) * (1.0 / 12.0);
+    S[3] += -0.5 * H20 - m[0][0] * (1.0 / 24.0) + (a * m[2][0] + b * m[1][1]) * (1.0 / 12.0);
+    S[4] += -0.5 * H02 - m[0][0] * (1.0 / 24.0) + (b * m[1][1] + c * m[0][2]) * (1.0 / 12.0);
+    S[5] += -H11 + (b * ((double)m[2][0] + m[0][2]) + t * m[1][1]) * (1.0 / 12.0);
+}
+#endif
 
 // Whether the region {E = dx^T F dx <= MAX_EXP_ARG (1% margin)} of a Gaussian
 // (FP32 pixel-loop parameters A = (xc, yc, c Fxx, c Fxy), fys = c Fyy) meets
@@ -619,7 +813,7 @@ __device__ __forceinline__ bool ellipse_meets_rect(const float4 A, float fys, fl
 }
 
 struct tile_smem {
-    size_t ga, gb, box, pix, wsrc, red, ints, keepw, idx, total;
+    size_t ga, gb, box, pix, wsrc, red, ints, rows, keepw, idx, total;
 };
 
 __host__ __device__ inline tile_smem tile_smem_layout(int tile_pixels, int max_gauss)
@@ -633,6 +827,7 @@ __host__ __device__ inline tile_smem tile_smem_layout(int tile_pixels, int max_g
     L.wsrc = o; o += (size_t)FP_WARPS * MAXSOURCES * NPARAMS * 8;
     L.red = o;  o += 16 * 8;
     L.ints = o; o += 32 * 4;
+    L.rows = o; o += 32 * 4;
     L.keepw = o; o += (((size_t)max_gauss + 31) / 32 * 4 + 15) & ~(size_t)15;
     L.idx = o;  o += ((size_t)max_gauss * 2 + 15) & ~(size_t)15;
     L.total = o;
@@ -667,6 +862,7 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
     int *s_int = reinterpret_cast<int *>(smem + L.ints);          // [0] item, [8..16) warp counts
     uint16_t *s_idx = reinterpret_cast<uint16_t *>(smem + L.idx);
     unsigned *s_keepw = reinterpret_cast<unsigned *>(smem + L.keepw); // cull ballot words
+    unsigned *s_rows = reinterpret_cast<unsigned *>(smem + L.rows);   // occupied places of the grid's rows
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool nocull = (flags & FP_FLAG_NO_CULL) != 0;
@@ -750,15 +946,20 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
         FP_PHASE_MARK(ph1);
         // ---- 2. forward: the tile's pixel class sets the pixels per thread ----
         int nzt;
+#ifdef FP_KAHAN
+        tile_grid grid = tile_grid_of(tl, ox, oy, false);
+#else
+        tile_grid grid = tile_grid_of(tl, ox, oy, !(flags & (FP_FLAG_FORWARD_ONLY | FP_FLAG_PIXEL_LIST)));
+#endif
         if (tl.tile_pixels == 1024)
             nzt = forward_tile<4>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, ox, oy, nocull, gc, s_idx, s_ga,
-                                  s_gb, s_gbox, s_pix, s_int, s_red);
+                                  s_gb, s_gbox, s_pix, s_int, s_red, s_rows, grid);
         else if (tl.tile_pixels == 512)
             nzt = forward_tile<2>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, ox, oy, nocull, gc, s_idx, s_ga,
-                                  s_gb, s_gbox, s_pix, s_int, s_red);
+                                  s_gb, s_gbox, s_pix, s_int, s_red, s_rows, grid);
         else
             nzt = forward_tile<1>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, ox, oy, nocull, gc, s_idx, s_ga,
-                                  s_gb, s_gbox, s_pix, s_int, s_red);
+                                  s_gb, s_gbox, s_pix, s_int, s_red, s_rows, grid);
         for (int t = tid; t < FP_WARPS * MAXSOURCES * NPARAMS; t += FP_THREADS) s_wsrc[t] = 0.0;
 
         FP_PHASE_MARK(ph2);
@@ -773,23 +974,33 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
                     s_gb[i] = gfwd[2 * gi + 1];
                 }
             }
-            // the (group of 32 Gaussians) x (pixel) plane, split evenly over the warps
+            // the (group of 32 Gaussians) x (unit) plane, split evenly over the
+            // warps: a unit is a pixel of the list, or a row of a strip of the grid
             __syncthreads();
             const int ngrp = (cn + 31) >> 5;
             const int vlast = cn - ((ngrp - 1) << 5);             // Gaussians in the last group
             const int krep = min(FP_MAX_REPLICAS, 32 / vlast);   // its replicas
-            const int ulast = (nzt + krep - 1) / krep;            // its units of krep pixels
-            // units of the (group, pixel) plane: at most 8 groups x 1024 pixels
-            const int ufull = (ngrp - 1) * nzt;
+            // units of a full group, and of the last one (krep pixels or rows each)
+            int nun = nzt, ulast = (nzt + krep - 1) / krep;
+            if (grid.on) {
+                nun = ulast = 0;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    nun += grid.strip[j] & 63;
+                    ulast += ((grid.strip[j] & 63) + krep - 1) / krep;
+                }
+            }
+            // at most 8 groups x 1024 units
+            const int ufull = (ngrp - 1) * nun;
             const int W = ufull + ulast;
             int u = W * warp / FP_WARPS;
             const int u1 = W * (warp + 1) / FP_WARPS;
             while (u < u1) {
                 int grp, q0, qn;
                 if (u < ufull) {
-                    grp = u / nzt;
-                    q0 = u - grp * nzt;
-                    qn = nzt;
+                    grp = u / nun;
+                    q0 = u - grp * nun;
+                    qn = nun;
                 } else {
                     grp = ngrp - 1;
                     q0 = u - ufull;
@@ -803,31 +1014,57 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
                 const bool valid = rep < kr && gl < cn;
                 const float4 A = valid ? s_ga[gl] : make_float4(0.f, 0.f, 0.f, 0.f);
                 const float4 B = valid ? s_gb[gl] : make_float4(0.f, 0.f, 0.f, 0.f);
-                double mom[12];
+                const int gidx = s_idx[c0 + (valid ? gl : 0)];
+                const double *J = gjac + (size_t)FP_JAC * (ed.gauss_offset + gidx);
+                double S[6];
 #pragma unroll
-                for (int k = 0; k < 12; ++k) mom[k] = 0.0;
-                if (kr == 1) {
-                    adjoint_moments<false>(A, B, s_pix, q0, q1, 1, mom);
-                } else {
-                    // replica rep takes pixels q*kr + rep of units [q0, q1): the
-                    // warp reads kr consecutive pixels per step
-                    const int pe = min(nzt, q1 * kr);
-                    adjoint_moments<true>(A, B, s_pix, valid ? q0 * kr + rep : pe, pe, kr, mom);
-                    // sum the replicas into replica 0 (lanes 0 .. vg-1), fixed tree
-                    for (int o = 1; o < kr; o <<= 1) {
-                        const bool take = (rep & (2 * o - 1)) == 0 && rep + o < kr;
+                for (int k = 0; k < 6; ++k) S[k] = 0.0;
+#ifndef FP_KAHAN
+                if (grid.on) {
+                    // units run down the rows of one strip, then the next; replica
+                    // rep takes rows rep, rep + kr, ...
+                    int first = 0;
+#pragma unroll 1
+                    for (int j = 0; j < 8 && first < q1; ++j) {
+                        const int st = s_int[16 + j], lo = st >> 6, nrow = st & 63;
+                        const int n = (nrow + kr - 1) / kr;
+                        const int b0 = max(q0 - first, 0), b1 = min(q1 - first, n);
+                        first += n;
+                        if (b0 >= b1) continue;
+                        const int rend = lo + min(nrow, b1 * kr);
+                        grid_partials(A, B, J, reinterpret_cast<const float *>(s_pix) + 4 * j,
+                                      valid ? lo + b0 * kr + rep : rend, rend, kr, grid.x0 + (float)(4 * j),
+                                      grid.y0, S);
+                    }
+                } else
+#endif
+                {
+                    double mom[12];
 #pragma unroll
-                        for (int k = 0; k < 12; ++k) {
-                            const double t = __shfl_down_sync(0xffffffffu, mom[k], o * vg);
-                            if (take) mom[k] += t;
-                        }
+                    for (int k = 0; k < 12; ++k) mom[k] = 0.0;
+                    if (kr == 1) {
+                        adjoint_moments<false>(A, B, s_pix, q0, q1, 1, mom);
+                    } else {
+                        // replica rep takes pixels q*kr + rep of units [q0, q1): the
+                        // warp reads kr consecutive pixels per step
+                        const int pe = min(nzt, q1 * kr);
+                        adjoint_moments<true>(A, B, s_pix, valid ? q0 * kr + rep : pe, pe, kr, mom);
+                    }
+                    moments_to_partials(J, mom, S);
+                }
+                // sum the replicas into replica 0 (lanes 0 .. vg-1), fixed tree
+                for (int o = 1; o < kr; o <<= 1) {
+                    const bool take = (rep & (2 * o - 1)) == 0 && rep + o < kr;
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) {
+                        const double t = __shfl_down_sync(0xffffffffu, S[k], o * vg);
+                        if (take) S[k] += t;
                     }
                 }
                 double g7[NPARAMS];
                 int src = -1;
                 if (valid && rep == 0) {
-                    const int gidx = s_idx[c0 + gl];
-                    moments_to_grad(gjac + (size_t)FP_JAC * (ed.gauss_offset + gidx), mom, g7);
+                    partials_to_grad(J, S, g7);
                     src = gidx / n_psf;               // Gaussian g belongs to source g / n_psf
                 } else {
 #pragma unroll
