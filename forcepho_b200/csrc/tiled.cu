@@ -17,12 +17,13 @@
 //                     E <= MAX_EXP_ARG ellipse (FP64), meets the tile's pixel
 //                     box; every other Gaussian has E > MAX_EXP_ARG at every
 //                     pixel of the tile and contributes exactly nothing;
-//                  2. forward, pixel-parallel: P pixels per thread, Gaussians
+//                  2. forward, pixel-parallel: 4 pixels per thread, Gaussians
 //                     staged in shared memory; per run of 32 Gaussians one box
 //                     test per lane and a warp ballot, the warp visiting only
 //                     the hits; y terms once per row of pixels; SFU ex2; FP32
-//                     runs flushed into per-pixel FP64 sums; residual, chi2
-//                     term in f64, w = r ierr^2;
+//                     runs flushed into per-pixel FP64 sums (tiles of fewer
+//                     than 1024 pixels: the runs are split over the warps);
+//                     residual, chi2 term in f64, w = r ierr^2;
 //                  3. adjoint, Gaussian-parallel: one Gaussian per lane.  The
 //                     tile's weights lie in shared memory as a dense grid of
 //                     its cell, walked down strips of 4 columns, or, where
@@ -270,24 +271,103 @@ __device__ __forceinline__ tile_grid tile_grid_of(const fp_tile &tl, const float
     return g;
 }
 
-// Forward pass of one tile, P pixels per thread (the tile holds at most
-// 256 P pixels): the model of each pixel over the tile's kept Gaussians, the
-// residual (written out when the patch has a residual array), the chi2 terms
-// reduced into s_red[FP_WARPS], and the nonzero-weight pixels (x, y, w) compacted
-// into s_pix in ascending order.  Returns their count (the same on every thread).
-// With s_rows, the weights go into the dense grid of grid_partials at s_pix
+// The staged Gaussians of a chunk, as the forward pass reads them: values that
+// multiply pairs of pixels are stored twice, ready for the packed instructions.
+struct staged_gauss {
+    fp_f4 *g0;      // (-xc, -xc), (c Fxx, c Fxx)
+    fp_f4 *g1;      // (c Fxy, c Fxy), (A C24, A C24)
+    fp_f4 *g2;      // (A k0, A k0), (yc, c Fyy)
+};
+
+__device__ __forceinline__ void stage(const staged_gauss &s, int i, const float4 *__restrict__ gfwd,
+                                      const float2 *__restrict__ gctr, int64_t gi, float ox, float oy)
+{
+    const float4 A = stage_gauss(gfwd, gctr, gi, ox, oy), B = gfwd[2 * gi + 1];
+    s.g0[i] = {fp_dup(-A.x), fp_dup(A.z)};
+    s.g1[i] = {fp_dup(A.w), fp_dup(B.z)};
+    s.g2[i] = {fp_dup(B.y), make_float2(A.y, B.x)};
+}
+
+// How a warp's pixels meet a Gaussian.  ROWS: every thread's 4 pixels lie in
+// one row, so the y terms are formed once per thread.  Otherwise they are
+// formed per pixel, with F dx's second component as c Fyy dy + fma'd c Fxy dx
+// (SAME_Y, the rounding of ROWS) or the other way round (ANY_Y); MIXED holds
+// pixels of both.  Which rounding a pixel gets is a matter of its place in its
+// tile alone (forward_tile), so that results do not depend on how the pixels
+// are spread over threads.
+enum forward_form { ROWS, SAME_Y, ANY_Y, MIXED };
+
+// Adds the run's Gaussians in `word` (bit i: s.g*[r0 + i]) to 4 pixels' FP32
+// sums, in ascending order.
+template <forward_form FORM>
+__device__ __forceinline__ void forward_run(unsigned word, int r0, const staged_gauss &s, const fp_f2 (&x)[2],
+                                            const fp_f2 (&y)[2], bool same_y, float (&m)[4], float (&mc)[4])
+{
+#pragma unroll 1
+    for (int i = r0; word != 0u; ++i, word >>= 1) {
+        if ((word & 1u) == 0u) continue;
+        const fp_f4 g0 = s.g0[i], g1 = s.g1[i], g2 = s.g2[i];
+        const float yc = g2.y.x, fyy = g2.y.y;
+        const float dy0 = y[0].x - yc;
+        const fp_f2 dyr = fp_dup(dy0), tyr = __fmul2_rn(g1.x, dyr), uyr = fp_dup(fyy * dy0);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const fp_f2 dx = __fadd2_rn(x[k], g0.x);
+            const fp_f2 dy = FORM == ROWS ? dyr : __fadd2_rn(y[k], fp_dup(-yc));
+            const fp_f2 vx = __ffma2_rn(g0.y, dx, FORM == ROWS ? tyr : __fmul2_rn(g1.x, dy));
+            fp_f2 vy;
+            if (FORM == ROWS) {
+                vy = __ffma2_rn(g1.x, dx, uyr);
+            } else {
+                const fp_f2 same = __ffma2_rn(g1.x, dx, __fmul2_rn(fp_dup(fyy), dy));
+                const fp_f2 any = __ffma2_rn(fp_dup(fyy), dy, __fmul2_rn(g1.x, dx));
+                vy = FORM == SAME_Y || (FORM == MIXED && same_y) ? same : any;
+            }
+            const fp_f2 e = __ffma2_rn(dy, vy, __fmul2_rn(dx, vx));
+            const fp_f2 h = __ffma2_rn(g1.y, __ffma2_rn(vx, vx, __fmul2_rn(vy, vy)), g2.x);
+            const float ga = fp_ex2(e.x), gb = fp_ex2(e.y);
+#ifdef FP_KAHAN
+            kahan_add(m[2 * k], mc[2 * k], (e.x < FP_CUT_SCALED) ? 0.f : ga * h.x);
+            kahan_add(m[2 * k + 1], mc[2 * k + 1], (e.y < FP_CUT_SCALED) ? 0.f : gb * h.y);
+#else
+            m[2 * k] = (e.x < FP_CUT_SCALED) ? m[2 * k] : fmaf(ga, h.x, m[2 * k]);
+            m[2 * k + 1] = (e.y < FP_CUT_SCALED) ? m[2 * k + 1] : fmaf(gb, h.y, m[2 * k + 1]);
+#endif
+        }
+    }
+}
+
+// Forward pass of one tile of class P (at most 256 P pixels): the model of each
+// pixel over the tile's kept Gaussians, the residual (written out when the
+// patch has a residual array), the chi2 terms reduced into s_red[FP_WARPS], and
+// the nonzero-weight pixels (x, y, w) compacted into s_pix in ascending order.
+// Returns their count (the same on every thread).
+// With grid.on, the weights go into the dense grid of grid_partials at s_pix
 // instead, if every weighted pixel has a place of its own there (grid.on is
-// then left true); x0, y0 are the relative coordinates of its first place.
+// then left true).
 // Pixel coordinates and Gaussian centres are taken relative to the tile's
 // origin (ox, oy) (stage_gauss); the boxes stay absolute.
+//
+// A thread holds 4 pixels, whatever the class: the 3 loads of a Gaussian, its
+// ballot bit and the row's y terms then cost a quarter each, and the pairs of
+// pixels share packed instructions.  A tile of fewer than 1024 pixels needs
+// only some of the warps for that; the others take other runs of 32 Gaussians
+// of the same pixels, and the runs' FP32 sums meet in FP64.
+// A packed operation on three different pairs takes 3 cycles of a scheduler's
+// register ports, not 2; at 13 such cycles per pixel with 8 of the SFU's they
+// bound the loop, which any mix of packed and scalar operations runs within 2 %.
+// Forward-only tile kernel with one pixel per thread in 256-pixel tiles, all
+// scalar, and as here: 58 and 46 us on a 16-source patch of 10 exposures of
+// 150x150 px (256-pixel tiles), 2.00 and 1.82 ms on 48 field patches.
+// s_m: 1024 doubles for those sums, free until the adjoint.
 template <int P>
 __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure_desc &ed, const fp_patch *pt,
                                             const int32_t *__restrict__ perm, const float4 *__restrict__ pix,
                                             const float4 *__restrict__ gfwd, const float4 *__restrict__ gbox,
                                             const float2 *__restrict__ gctr, const float ox, const float oy,
-                                            const bool nocull, const int gc, const uint16_t *s_idx, float4 *s_ga,
-                                            float4 *s_gb, float4 *s_gbox, float4 *s_pix, int *s_int, double *s_red,
-                                            unsigned *s_rows, tile_grid &grid)
+                                            const bool nocull, const int gc, const uint16_t *s_idx,
+                                            const staged_gauss &sg, float4 *s_gbox, float4 *s_pix, int *s_int,
+                                            double *s_red, double *s_m, unsigned *s_rows, tile_grid &grid)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int npix = tl.n_pix;
@@ -298,148 +378,147 @@ __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure
         if (tid < 32) s_rows[tid] = 0u;
     }
 
-    // the tile's pixels are listed in the plan's pixel order (compact cells)
-    const int j0 = tid * P;
-    const int nval = npix - j0;
-    const int32_t *tperm = perm + tl.perm_start + j0;
-    int idx[P];
-    float xs[P], ys[P], ds[P], es[P];
-    if (pix != nullptr) {
-        // contiguous (x, y, data, ierr) records in plan order: one 16-byte
-        // load per pixel; the patch index only where a residual is written
-        const float4 *rec = pix + tl.perm_start + j0;
-        const bool want_idx = pt->residual != nullptr;
+    // warps per set of the tile's pixels, and the sets; each set takes every
+    // sets-th run of Gaussians
+    const int per_set = npix > 512 ? 8 : npix > 256 ? 4 : npix > 128 ? 2 : 1;
+    const int sets = FP_WARPS / per_set, set = warp / per_set;
+    double M[4] = {0.0, 0.0, 0.0, 0.0};
+#ifdef FP_KAHAN
+    float ms[4] = {0.f, 0.f, 0.f, 0.f}, mc[4] = {0.f, 0.f, 0.f, 0.f};   // per-pixel compensated FP32 model sums
+#endif
+    {
+        // the tile's pixels are listed in the plan's pixel order (compact cells)
+        const int j0 = 4 * ((warp % per_set) * 32 + lane), nval = npix - j0;
+        float xs[4], ys[4];
         const uint64_t pol = fp_policy_evict_first();
 #pragma unroll
-        for (int k = 0; k < P; ++k) {
-            const float4 r = (k < nval) ? fp_ldg_policy(rec + k, pol) : make_float4(0.f, 0.f, 0.f, 0.f);
-            xs[k] = r.x; ys[k] = r.y; ds[k] = r.z; es[k] = r.w;
-            idx[k] = (k < nval && want_idx) ? __ldg(tperm + k) : -1;
+        for (int k = 0; k < 4; ++k) {
+            xs[k] = ys[k] = 0.f;
+            if (k < nval) {
+                if (pix != nullptr) {
+                    const float4 r = fp_ldg_policy(pix + tl.perm_start + j0 + k, pol);
+                    xs[k] = r.x;
+                    ys[k] = r.y;
+                } else {
+                    const int32_t ix = __ldg(perm + tl.perm_start + j0 + k);
+                    xs[k] = __ldg(pt->xpix + ix);
+                    ys[k] = __ldg(pt->ypix + ix);
+                }
+            }
         }
-    } else {
+        // this warp's pixel box: Gaussians whose box misses it are skipped by
+        // the whole warp (they have E > MAX_EXP_ARG at all of its pixels)
+        float wx0 = INFINITY, wx1 = -INFINITY, wy0 = INFINITY, wy1 = -INFINITY;
 #pragma unroll
-        for (int k = 0; k < P; ++k) {
-            idx[k] = (k < nval) ? __ldg(tperm + k) : -1;
-            const bool ok = idx[k] >= 0;
-            xs[k] = ok ? __ldg(pt->xpix + idx[k]) : 0.f;
-            ys[k] = ok ? __ldg(pt->ypix + idx[k]) : 0.f;
-            ds[k] = ok ? __ldg(pt->data + idx[k]) : 0.f;
-            es[k] = ok ? __ldg(pt->ierr + idx[k]) : 0.f;
+        for (int k = 0; k < 4; ++k)
+            if (k < nval) {
+                wx0 = fminf(wx0, xs[k]); wx1 = fmaxf(wx1, xs[k]);
+                wy0 = fminf(wy0, ys[k]); wy1 = fmaxf(wy1, ys[k]);
+            }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            wx0 = fminf(wx0, __shfl_xor_sync(0xffffffffu, wx0, o));
+            wx1 = fmaxf(wx1, __shfl_xor_sync(0xffffffffu, wx1, o));
+            wy0 = fminf(wy0, __shfl_xor_sync(0xffffffffu, wy0, o));
+            wy1 = fmaxf(wy1, __shfl_xor_sync(0xffffffffu, wy1, o));
         }
-    }
-    // this warp's pixel box: Gaussians whose box misses it are skipped by
-    // the whole warp (they have E > MAX_EXP_ARG at all of its pixels)
-    float wx0 = INFINITY, wx1 = -INFINITY, wy0 = INFINITY, wy1 = -INFINITY;
+        if (nocull) { wx0 = wy0 = -INFINITY; wx1 = wy1 = INFINITY; }
 #pragma unroll
-    for (int k = 0; k < P; ++k)
-        if (k < nval) {
-            wx0 = fminf(wx0, xs[k]); wx1 = fmaxf(wx1, xs[k]);
-            wy0 = fminf(wy0, ys[k]); wy1 = fmaxf(wy1, ys[k]);
+        for (int k = 0; k < 4; ++k) {
+            xs[k] -= ox;
+            ys[k] -= oy;
         }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        wx0 = fminf(wx0, __shfl_xor_sync(0xffffffffu, wx0, o));
-        wx1 = fmaxf(wx1, __shfl_xor_sync(0xffffffffu, wx1, o));
-        wy0 = fminf(wy0, __shfl_xor_sync(0xffffffffu, wy0, o));
-        wy1 = fmaxf(wy1, __shfl_xor_sync(0xffffffffu, wy1, o));
-    }
-    if (nocull) { wx0 = wy0 = -INFINITY; wx1 = wy1 = INFINITY; }
-#pragma unroll
-    for (int k = 0; k < P; ++k) {
-        xs[k] -= ox;
-        ys[k] -= oy;
-    }
-    // one row: every thread's pixels share their y (cell rows in row order),
-    // so the y-dependent products of a Gaussian are formed once per thread
-    bool same_y = true;
-#pragma unroll
-    for (int k = 1; k < P; ++k) same_y = same_y && (k >= nval || ys[k] == ys[0]);
-    const bool rowwise = __all_sync(0xffffffffu, same_y);
-#ifdef FP_KAHAN
-    float KS[P], KC[P];     // per-pixel compensated FP32 model sums
-#pragma unroll
-    for (int k = 0; k < P; ++k) KS[k] = KC[k] = 0.f;
-#else
-    double M[P];
-#pragma unroll
-    for (int k = 0; k < P; ++k) M[k] = 0.0;
-#endif
+        // a pixel has the SAME_Y rounding if, over its segment of 32 P pixels of
+        // the tile, every P consecutive pixels from the tile's first share a row
+        const bool y01 = 1 >= nval || ys[1] == ys[0], y23 = 3 >= nval || ys[3] == ys[2];
+        const bool row4 = y01 && (2 >= nval || ys[2] == ys[0]) && (3 >= nval || ys[3] == ys[0]);
+        const bool rows = __all_sync(0xffffffffu, row4);
+        bool same_y = P == 1 || (P == 4 && rows);
+        if (P == 2) {
+            const unsigned pairs = __ballot_sync(0xffffffffu, y01 && y23);
+            same_y = ((pairs >> (lane & 16)) & 0xffffu) == 0xffffu;
+        }
+        const forward_form form = rows ? ROWS
+                                       : __all_sync(0xffffffffu, same_y) ? SAME_Y
+                                       : __any_sync(0xffffffffu, same_y) ? MIXED : ANY_Y;
+        const fp_f2 x[2] = {make_float2(xs[0], xs[1]), make_float2(xs[2], xs[3])};
+        const fp_f2 y[2] = {make_float2(ys[0], ys[1]), make_float2(ys[2], ys[3])};
 
-    for (int c0 = 0; c0 < gc; c0 += FP_CHUNK) {
-        const int cn = min(FP_CHUNK, gc - c0);
-        __syncthreads();
-        for (int i = tid; i < cn; i += FP_THREADS) {
-            const int64_t gi = ed.gauss_offset + s_idx[c0 + i];
-            s_ga[i] = stage_gauss(gfwd, gctr, gi, ox, oy);
-            s_gb[i] = gfwd[2 * gi + 1];
-            s_gbox[i] = gbox[gi];
-        }
-        __syncthreads();
-        {
+        for (int c0 = 0; c0 < gc; c0 += FP_CHUNK) {
+            const int cn = min(FP_CHUNK, gc - c0);
+            __syncthreads();
+            for (int i = tid; i < cn; i += FP_THREADS) {
+                const int64_t gi = ed.gauss_offset + s_idx[c0 + i];
+                stage(sg, i, gfwd, gctr, gi, ox, oy);
+                s_gbox[i] = gbox[gi];
+            }
+            __syncthreads();
             // runs of 32 Gaussians: lane l tests Gaussian r0 + l against the
             // warp's pixel box, and the warp visits the hits of the run in
             // ascending order; each run is summed in FP32, then added in FP64.
             // Every lane takes part in the ballot, including lanes without
             // pixels (their sums are never used).
-            for (int r0 = 0; r0 < cn; r0 += 32) {
+            for (int r0 = 32 * set; r0 < cn; r0 += 32 * sets) {
                 const int il = r0 + lane;
                 bool hit = false;
                 if (il < cn) {
                     const float4 bx = s_gbox[il];
                     hit = !(bx.y < wx0 || bx.x > wx1 || bx.w < wy0 || bx.z > wy1);
                 }
-                unsigned word = __ballot_sync(0xffffffffu, hit);
-                float m[P];
-#pragma unroll
-                for (int k = 0; k < P; ++k) m[k] = 0.f;
-                if (rowwise) {
-                    while (word) {
-                        const int i = r0 + __ffs(word) - 1;
-                        word &= word - 1u;
-                        const float4 A = s_ga[i], B = s_gb[i];
-                        const float dy = ys[0] - A.y;
-                        const float ty = A.w * dy, uy = B.x * dy;     // c Fxy dy, c Fyy dy
-#pragma unroll
-                        for (int k = 0; k < P; ++k) {
-                            const float dx = xs[k] - A.x;
-                            const float vx = fmaf(A.z, dx, ty);
-                            const float vy = fmaf(A.w, dx, uy);
-                            const float e = fmaf(dy, vy, dx * vx);
-                            const float g = fp_ex2(e);
-                            const float h = fmaf(B.z, fmaf(vx, vx, vy * vy), B.y);
-#ifdef FP_KAHAN
-                            kahan_add(KS[k], KC[k], (e < FP_CUT_SCALED) ? 0.f : g * h);
-#else
-                            m[k] = (e < FP_CUT_SCALED) ? m[k] : fmaf(g, h, m[k]);
+                const unsigned word = __ballot_sync(0xffffffffu, hit);
+#ifndef FP_KAHAN
+                float ms[4] = {0.f, 0.f, 0.f, 0.f}, mc[4];
 #endif
-                        }
-                    }
-                } else {
-                    while (word) {
-                        const int i = r0 + __ffs(word) - 1;
-                        word &= word - 1u;
-                        const float4 A = s_ga[i], B = s_gb[i];
-#pragma unroll
-                        for (int k = 0; k < P; ++k) {
-                            const float dx = xs[k] - A.x, dy = ys[k] - A.y;
-                            const float vx = fmaf(A.z, dx, A.w * dy);
-                            const float vy = fmaf(B.x, dy, A.w * dx);
-                            const float e = fmaf(dy, vy, dx * vx);
-                            const float g = fp_ex2(e);
-                            const float h = fmaf(B.z, fmaf(vx, vx, vy * vy), B.y);
-#ifdef FP_KAHAN
-                            kahan_add(KS[k], KC[k], (e < FP_CUT_SCALED) ? 0.f : g * h);
-#else
-                            m[k] = (e < FP_CUT_SCALED) ? m[k] : fmaf(g, h, m[k]);
-#endif
-                        }
-                    }
-                }
+                if (form == ROWS) forward_run<ROWS>(word, r0, sg, x, y, same_y, ms, mc);
+                else if (form == ANY_Y) forward_run<ANY_Y>(word, r0, sg, x, y, same_y, ms, mc);
+                else if (form == SAME_Y) forward_run<SAME_Y>(word, r0, sg, x, y, same_y, ms, mc);
+                else forward_run<MIXED>(word, r0, sg, x, y, same_y, ms, mc);
 #ifndef FP_KAHAN
 #pragma unroll
-                for (int k = 0; k < P; ++k) M[k] += (double)m[k];
+                for (int k = 0; k < 4; ++k) M[k] += (double)ms[k];
 #endif
             }
+        }
+#ifdef FP_KAHAN
+#pragma unroll
+        for (int k = 0; k < 4; ++k) M[k] = (double)ms[k] - (double)mc[k];
+#endif
+        if (P != 4 || sets > 1) {
+            double *mine = s_m + 128 * per_set * set + j0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) mine[k] = M[k];
+        }
+    }
+
+    // from here a thread holds P pixels
+    const int j0 = tid * P, nval = npix - j0;
+    int idx[P];
+    float xs[P], ys[P], ds[P], es[P];
+    {
+        const bool want_idx = pix == nullptr || pt->residual != nullptr;
+        const uint64_t pol = fp_policy_evict_first();
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+            const bool live = k < nval;
+            idx[k] = (live && want_idx) ? __ldg(perm + tl.perm_start + j0 + k) : -1;
+            float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (live) {
+                if (pix != nullptr)
+                    r = fp_ldg_policy(pix + tl.perm_start + j0 + k, pol);
+                else
+                    r = make_float4(__ldg(pt->xpix + idx[k]), __ldg(pt->ypix + idx[k]), __ldg(pt->data + idx[k]),
+                                    __ldg(pt->ierr + idx[k]));
+            }
+            xs[k] = r.x - ox; ys[k] = r.y - oy; ds[k] = r.z; es[k] = r.w;
+        }
+    }
+    if (P != 4 || sets > 1) {
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+            M[k] = 0.0;
+            if (k < nval)
+                for (int g = 0; g < sets; ++g) M[k] += s_m[128 * per_set * g + j0 + k];
         }
     }
 
@@ -454,7 +533,7 @@ __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure
     for (int k = 0; k < P; ++k) {
         const bool live = k < nval;
 #ifdef FP_KAHAN
-        const float r = ds[k] - (KS[k] - KC[k]);
+        const float r = ds[k] - (float)M[k];
         rs[k] = r;
         const float rif = r * es[k], dif = ds[k] * es[k];
         kahan_add(chi_s, chi_c, live ? (rif - dif) * (rif + dif) : 0.f);
@@ -565,11 +644,11 @@ __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure
 // libforcepho_b200_kahan.so): every moment summed over the whole pixel range
 // in FP32 with a compensation term, converted to FP64 once at the end.
 template <bool STRIDED>
-__device__ __forceinline__ void adjoint_moments(const float4 A, const float4 B,
+__device__ __forceinline__ void adjoint_moments(const float4 A, const float fys, const float k0,
                                                 const float4 *__restrict__ s_pix, int p0, int p1, int k,
                                                 double (&m)[12])
 {
-    const float xc = A.x, yc = A.y, fxs = A.z, fxys = A.w, fys = B.x, k0 = B.w;
+    const float xc = A.x, yc = A.y, fxs = A.z, fxys = A.w;
     const float c24 = (float)FP_C24;
     const int step = STRIDED ? k : 1;
     float a[12], c[12];
@@ -604,11 +683,11 @@ __device__ __forceinline__ void adjoint_moments(const float4 A, const float4 B,
 }
 #else
 template <bool STRIDED>
-__device__ __forceinline__ void adjoint_moments(const float4 A, const float4 B,
+__device__ __forceinline__ void adjoint_moments(const float4 A, const float fys, const float k0,
                                                 const float4 *__restrict__ s_pix, int p0, int p1, int k,
                                                 double (&m)[12])
 {
-    const float xc = A.x, yc = A.y, fxs = A.z, fxys = A.w, fys = B.x, k0 = B.w;
+    const float xc = A.x, yc = A.y, fxs = A.z, fxys = A.w;
     const float c24 = (float)FP_C24;
     const int step = STRIDED ? k : 1;
     for (int r0 = p0; r0 < p1; r0 += FP_RUN * step) {
@@ -706,7 +785,7 @@ __device__ __forceinline__ void partials_to_grad(const double *__restrict__ J, c
 // Tile kernel on 48 field patches (2.9e9 evaluated pairs): 6.31 ms with the
 // list, 4.02 ms here; on a 30-source patch of 32 exposures of 256x256 px,
 // 1.64 and 0.98 ms.
-__device__ __forceinline__ void grid_partials(const float4 A, const float4 B, const double *__restrict__ J,
+__device__ __forceinline__ void grid_partials(const float4 A, float Fyy, const double *__restrict__ J,
                                               const float *__restrict__ s_w, int r, int rend, int step, float x,
                                               float y0, double (&S)[6])
 {
@@ -714,7 +793,7 @@ __device__ __forceinline__ void grid_partials(const float4 A, const float4 B, co
 #pragma unroll
     for (int k = 0; k < 4; ++k) dx[k] = (x + (float)k) - A.x;
     {
-        const fp_f2 nyc = fp_dup(-A.y), fyy = fp_dup(B.x), ystep = fp_dup((float)step);
+        const fp_f2 nyc = fp_dup(-A.y), fyy = fp_dup(Fyy), ystep = fp_dup((float)step);
         fp_f2 y = fp_dup(y0 + (float)r);
         fp_f2 l[2], q[2], Y[5][2];
 #pragma unroll
@@ -813,15 +892,14 @@ __device__ __forceinline__ bool ellipse_meets_rect(const float4 A, float fys, fl
 }
 
 struct tile_smem {
-    size_t ga, gb, box, pix, wsrc, red, ints, rows, keepw, idx, total;
+    size_t g, box, pix, wsrc, red, ints, rows, keepw, idx, total;
 };
 
 __host__ __device__ inline tile_smem tile_smem_layout(int tile_pixels, int max_gauss)
 {
     tile_smem L;
     size_t o = 0;
-    L.ga = o;   o += (size_t)FP_CHUNK * 16;
-    L.gb = o;   o += (size_t)FP_CHUNK * 16;
+    L.g = o;    o += (size_t)FP_CHUNK * 3 * sizeof(fp_f4);
     L.box = o;  o += (size_t)FP_CHUNK * 16;
     L.pix = o;  o += (size_t)tile_pixels * 16;
     L.wsrc = o; o += (size_t)FP_WARPS * MAXSOURCES * NPARAMS * 8;
@@ -851,8 +929,8 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
     constexpr int T = FP_THREADS * P;
     extern __shared__ __align__(16) unsigned char smem[];
     const tile_smem L = tile_smem_layout(T, max_gauss);
-    float4 *s_ga = reinterpret_cast<float4 *>(smem + L.ga);
-    float4 *s_gb = reinterpret_cast<float4 *>(smem + L.gb);
+    fp_f4 *s_g = reinterpret_cast<fp_f4 *>(smem + L.g);
+    const staged_gauss sg = {s_g, s_g + FP_CHUNK, s_g + 2 * FP_CHUNK};
     float4 *s_gbox = reinterpret_cast<float4 *>(smem + L.box);
     float4 *s_pix = reinterpret_cast<float4 *>(smem + L.pix);
     // per-warp source gradients [warp][source][param]: each warp adds its own
@@ -952,14 +1030,14 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
         tile_grid grid = tile_grid_of(tl, ox, oy, !(flags & (FP_FLAG_FORWARD_ONLY | FP_FLAG_PIXEL_LIST)));
 #endif
         if (tl.tile_pixels == 1024)
-            nzt = forward_tile<4>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, ox, oy, nocull, gc, s_idx, s_ga,
-                                  s_gb, s_gbox, s_pix, s_int, s_red, s_rows, grid);
+            nzt = forward_tile<4>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, ox, oy, nocull, gc, s_idx, sg, s_gbox, s_pix,
+                                  s_int, s_red, s_wsrc, s_rows, grid);
         else if (tl.tile_pixels == 512)
-            nzt = forward_tile<2>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, ox, oy, nocull, gc, s_idx, s_ga,
-                                  s_gb, s_gbox, s_pix, s_int, s_red, s_rows, grid);
+            nzt = forward_tile<2>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, ox, oy, nocull, gc, s_idx, sg, s_gbox, s_pix,
+                                  s_int, s_red, s_wsrc, s_rows, grid);
         else
-            nzt = forward_tile<1>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, ox, oy, nocull, gc, s_idx, s_ga,
-                                  s_gb, s_gbox, s_pix, s_int, s_red, s_rows, grid);
+            nzt = forward_tile<1>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, ox, oy, nocull, gc, s_idx, sg, s_gbox, s_pix,
+                                  s_int, s_red, s_wsrc, s_rows, grid);
         for (int t = tid; t < FP_WARPS * MAXSOURCES * NPARAMS; t += FP_THREADS) s_wsrc[t] = 0.0;
 
         FP_PHASE_MARK(ph2);
@@ -970,8 +1048,7 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
             if (gc > FP_CHUNK) {
                 for (int i = tid; i < cn; i += FP_THREADS) {
                     const int64_t gi = ed.gauss_offset + s_idx[c0 + i];
-                    s_ga[i] = stage_gauss(gfwd, gctr, gi, ox, oy);
-                    s_gb[i] = gfwd[2 * gi + 1];
+                    stage(sg, i, gfwd, gctr, gi, ox, oy);
                 }
             }
             // the (group of 32 Gaussians) x (unit) plane, split evenly over the
@@ -1012,8 +1089,14 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
                 const int rep = lane / vg;
                 const int gl = grp * 32 + lane - rep * vg;
                 const bool valid = rep < kr && gl < cn;
-                const float4 A = valid ? s_ga[gl] : make_float4(0.f, 0.f, 0.f, 0.f);
-                const float4 B = valid ? s_gb[gl] : make_float4(0.f, 0.f, 0.f, 0.f);
+                float4 A = make_float4(0.f, 0.f, 0.f, 0.f);          // (xc, yc, c Fxx, c Fxy)
+                float fyy = 0.f;
+                if (valid) {
+                    const fp_f4 g0 = sg.g0[gl];
+                    const fp_f2 yf = sg.g2[gl].y;
+                    A = make_float4(-g0.x.x, yf.x, g0.y.x, sg.g1[gl].x.x);
+                    fyy = yf.y;
+                }
                 const int gidx = s_idx[c0 + (valid ? gl : 0)];
                 const double *J = gjac + (size_t)FP_JAC * (ed.gauss_offset + gidx);
                 double S[6];
@@ -1032,23 +1115,24 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
                         first += n;
                         if (b0 >= b1) continue;
                         const int rend = lo + min(nrow, b1 * kr);
-                        grid_partials(A, B, J, reinterpret_cast<const float *>(s_pix) + 4 * j,
+                        grid_partials(A, fyy, J, reinterpret_cast<const float *>(s_pix) + 4 * j,
                                       valid ? lo + b0 * kr + rep : rend, rend, kr, grid.x0 + (float)(4 * j),
                                       grid.y0, S);
                     }
                 } else
 #endif
                 {
+                    const float k0 = gfwd[2 * (ed.gauss_offset + gidx) + 1].w;
                     double mom[12];
 #pragma unroll
                     for (int k = 0; k < 12; ++k) mom[k] = 0.0;
                     if (kr == 1) {
-                        adjoint_moments<false>(A, B, s_pix, q0, q1, 1, mom);
+                        adjoint_moments<false>(A, fyy, k0, s_pix, q0, q1, 1, mom);
                     } else {
                         // replica rep takes pixels q*kr + rep of units [q0, q1): the
                         // warp reads kr consecutive pixels per step
                         const int pe = min(nzt, q1 * kr);
-                        adjoint_moments<true>(A, B, s_pix, valid ? q0 * kr + rep : pe, pe, kr, mom);
+                        adjoint_moments<true>(A, fyy, k0, s_pix, valid ? q0 * kr + rep : pe, pe, kr, mom);
                     }
                     moments_to_partials(J, mom, S);
                 }
