@@ -32,9 +32,9 @@ int fp_sm_count(int *out);
 // gauss_fwd  float4[2*n_gauss]    : (xc, yc, c fxx, c fxy), (c fyy, amp k0, amp C24, k0)
 // gauss_box  float4[n_gauss]      : xmin, xmax, ymin, ymax of the E <= 36 box
 // gauss_ctr  float2[n_gauss]      : xc - (float)xc, yc - (float)yc: what the FP32 centre lost
-// gauss_jac  double[FP_JAC*n_gauss]
+// gauss_jac  double[FP_JAC][n_gauss]
 // partials   double[n_partials]
-#define FP_JAC 20                   // amp, fxx, fxy, fyy, 15 Jacobian terms, pad
+#define FP_JAC 19                   // amp, fxx, fxy, fyy, 15 Jacobian terms
 struct fp_control {
     unsigned long long queue;       // next work item of the persistent tile kernel
     int status;                     // FP_STATUS_* bits
