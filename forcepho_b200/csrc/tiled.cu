@@ -103,6 +103,7 @@ setup_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc
              float4 *__restrict__ gbox, float2 *__restrict__ gctr, double *__restrict__ gjac, int64_t n_gauss,
              fp_control *ctl)
 {
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) ctl->queue = 0ULL;
     const fp_exposure_desc ed = expos[blockIdx.x];
     const int g = blockIdx.y * SETUP_THREADS + threadIdx.x;
     if (g > 0 && g >= ed.n_gauss) return;
@@ -389,6 +390,32 @@ __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure
         if (tid < 32) s_rows[tid] = 0u;
     }
 
+    // what the residual needs: P pixels of this thread, in the tile's order.
+    // Loaded ahead of the pass where few registers hold them (P < 4), so that
+    // small tiles do not wait for memory twice.
+    const int j0 = tid * P, nval = npix - j0;
+    int idx[P];
+    float xs[P], ys[P], ds[P], es[P];
+    const auto load = [&]() {
+        const bool want_idx = pix == nullptr || pt->residual != nullptr;
+        const uint64_t pol = fp_policy_evict_first();
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+            const bool live = k < nval;
+            idx[k] = (live && want_idx) ? __ldg(perm + tl.perm_start + j0 + k) : -1;
+            float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (live) {
+                if (pix != nullptr)
+                    r = fp_ldg_policy(pix + tl.perm_start + j0 + k, pol);
+                else
+                    r = make_float4(__ldg(pt->xpix + idx[k]), __ldg(pt->ypix + idx[k]), __ldg(pt->data + idx[k]),
+                                    __ldg(pt->ierr + idx[k]));
+            }
+            xs[k] = r.x - ox; ys[k] = r.y - oy; ds[k] = r.z; es[k] = r.w;
+        }
+    };
+    if (P < 4) load();
+
     // warps per set of the tile's pixels, and the sets; each set takes every
     // sets-th run of Gaussians
     const int per_set = npix > 512 ? 8 : npix > 256 ? 4 : npix > 128 ? 2 : 1;
@@ -399,21 +426,21 @@ __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure
 #endif
     {
         // the tile's pixels are listed in the plan's pixel order (compact cells)
-        const int j0 = 4 * ((warp % per_set) * 32 + lane), nval = npix - j0;
-        float xs[4], ys[4];
+        const int f0 = 4 * ((warp % per_set) * 32 + lane), fval = npix - f0;
+        float fx[4], fy[4];
         const uint64_t pol = fp_policy_evict_first();
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            xs[k] = ys[k] = 0.f;
-            if (k < nval) {
+            fx[k] = fy[k] = 0.f;
+            if (k < fval) {
                 if (pix != nullptr) {
-                    const float4 r = fp_ldg_policy(pix + tl.perm_start + j0 + k, pol);
-                    xs[k] = r.x;
-                    ys[k] = r.y;
+                    const float4 r = fp_ldg_policy(pix + tl.perm_start + f0 + k, pol);
+                    fx[k] = r.x;
+                    fy[k] = r.y;
                 } else {
-                    const int32_t ix = __ldg(perm + tl.perm_start + j0 + k);
-                    xs[k] = __ldg(pt->xpix + ix);
-                    ys[k] = __ldg(pt->ypix + ix);
+                    const int32_t ix = __ldg(perm + tl.perm_start + f0 + k);
+                    fx[k] = __ldg(pt->xpix + ix);
+                    fy[k] = __ldg(pt->ypix + ix);
                 }
             }
         }
@@ -422,9 +449,9 @@ __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure
         float wx0 = INFINITY, wx1 = -INFINITY, wy0 = INFINITY, wy1 = -INFINITY;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if (k < nval) {
-                wx0 = fminf(wx0, xs[k]); wx1 = fmaxf(wx1, xs[k]);
-                wy0 = fminf(wy0, ys[k]); wy1 = fmaxf(wy1, ys[k]);
+            if (k < fval) {
+                wx0 = fminf(wx0, fx[k]); wx1 = fmaxf(wx1, fx[k]);
+                wy0 = fminf(wy0, fy[k]); wy1 = fmaxf(wy1, fy[k]);
             }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -436,13 +463,13 @@ __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure
         if (nocull) { wx0 = wy0 = -INFINITY; wx1 = wy1 = INFINITY; }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            xs[k] -= ox;
-            ys[k] -= oy;
+            fx[k] -= ox;
+            fy[k] -= oy;
         }
         // a pixel has the SAME_Y rounding if, over its segment of 32 P pixels of
         // the tile, every P consecutive pixels from the tile's first share a row
-        const bool y01 = 1 >= nval || ys[1] == ys[0], y23 = 3 >= nval || ys[3] == ys[2];
-        const bool row4 = y01 && (2 >= nval || ys[2] == ys[0]) && (3 >= nval || ys[3] == ys[0]);
+        const bool y01 = 1 >= fval || fy[1] == fy[0], y23 = 3 >= fval || fy[3] == fy[2];
+        const bool row4 = y01 && (2 >= fval || fy[2] == fy[0]) && (3 >= fval || fy[3] == fy[0]);
         const bool rows = __all_sync(0xffffffffu, row4);
         bool same_y = P == 1 || (P == 4 && rows);
         if (P == 2) {
@@ -452,8 +479,8 @@ __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure
         const forward_form form = rows ? ROWS
                                        : __all_sync(0xffffffffu, same_y) ? SAME_Y
                                        : __any_sync(0xffffffffu, same_y) ? MIXED : ANY_Y;
-        const fp_f2 x[2] = {make_float2(xs[0], xs[1]), make_float2(xs[2], xs[3])};
-        const fp_f2 y[2] = {make_float2(ys[0], ys[1]), make_float2(ys[2], ys[3])};
+        const fp_f2 x[2] = {make_float2(fx[0], fx[1]), make_float2(fx[2], fx[3])};
+        const fp_f2 y[2] = {make_float2(fy[0], fy[1]), make_float2(fy[2], fy[3])};
 
         for (int c0 = 0; c0 < gc; c0 += FP_CHUNK) {
             const int cn = min(FP_CHUNK, gc - c0);
@@ -495,34 +522,14 @@ __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure
         for (int k = 0; k < 4; ++k) M[k] = (double)ms[k] - (double)mc[k];
 #endif
         if (P != 4 || sets > 1) {
-            double *mine = s_m + 128 * per_set * set + j0;
+            double *mine = s_m + 128 * per_set * set + f0;
 #pragma unroll
             for (int k = 0; k < 4; ++k) mine[k] = M[k];
         }
     }
 
     // from here a thread holds P pixels
-    const int j0 = tid * P, nval = npix - j0;
-    int idx[P];
-    float xs[P], ys[P], ds[P], es[P];
-    {
-        const bool want_idx = pix == nullptr || pt->residual != nullptr;
-        const uint64_t pol = fp_policy_evict_first();
-#pragma unroll
-        for (int k = 0; k < P; ++k) {
-            const bool live = k < nval;
-            idx[k] = (live && want_idx) ? __ldg(perm + tl.perm_start + j0 + k) : -1;
-            float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (live) {
-                if (pix != nullptr)
-                    r = fp_ldg_policy(pix + tl.perm_start + j0 + k, pol);
-                else
-                    r = make_float4(__ldg(pt->xpix + idx[k]), __ldg(pt->ypix + idx[k]), __ldg(pt->data + idx[k]),
-                                    __ldg(pt->ierr + idx[k]));
-            }
-            xs[k] = r.x - ox; ys[k] = r.y - oy; ds[k] = r.z; es[k] = r.w;
-        }
-    }
+    if (P == 4) load();
     if (P != 4 || sets > 1) {
         __syncthreads();
 #pragma unroll
@@ -957,12 +964,14 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
     const bool nocull = (flags & FP_FLAG_NO_CULL) != 0;
     const bool forward_only = (flags & FP_FLAG_FORWARD_ONLY) != 0;
 
+    // a CTA's first tile is its own number, the queue hands out the rest (none
+    // if every tile has a CTA: no atomic at all then)
     for (int64_t iter = 0;; ++iter) {
         if (tid == 0) {
-            const unsigned long long it = (flags & FP_FLAG_STATIC)
-                                              ? (unsigned long long)(blockIdx.x + iter * gridDim.x)
-                                              : atomicAdd(&ctl->queue, 1ULL);
-            s_int[0] = (it < (unsigned long long)n_tiles) ? order[it] : -1;
+            int64_t it = blockIdx.x + iter * gridDim.x;
+            if (iter > 0 && !(flags & FP_FLAG_STATIC))
+                it = n_tiles > gridDim.x ? gridDim.x + (int64_t)atomicAdd(&ctl->queue, 1ULL) : n_tiles;
+            s_int[0] = it < n_tiles ? order[it] : -1;
         }
         __syncthreads();
         const int ti = s_int[0];
@@ -1505,9 +1514,10 @@ int run_batch(const batch_launch &a, const fp_patch *const *d_patches, const fp_
         const int cps = launch->ctas_per_sm > 0 ? launch->ctas_per_sm : 2;
         const int64_t want = (int64_t)cps * a.n_sm;
         const int grid = (int)(want < sizes->n_tiles ? want : sizes->n_tiles);
-        // the persistent CTAs pop tiles from this counter
-        if (int rc = fp_check_cuda(cudaMemsetAsync(&ctl->queue, 0, sizeof(ctl->queue), st), "queue reset"))
-            return rc;
+        // the persistent CTAs pop tiles from this counter, which the setup resets
+        if (!((phases & FP_PHASE_SETUP) && sizes->n_exposures > 0))
+            if (int rc = fp_check_cuda(cudaMemsetAsync(&ctl->queue, 0, sizeof(ctl->queue), st), "queue reset"))
+                return rc;
         int rc;
         const int mg = (int)sizes->max_gauss;
         const int64_t ng = sizes->n_gauss;
