@@ -91,6 +91,7 @@ tile_dtype = np.dtype([("partial_offset", np.int64), ("expo", np.int32), ("perm_
                        ("n_pix", np.int32), ("tile_pixels", np.int32), ("bbox", np.float32, 4)])
 band_desc_dtype = np.dtype([("patch", np.int32), ("band", np.int32), ("tile_begin", np.int32),
                             ("tile_end", np.int32), ("n_sources", np.int32), ("pad", np.int32)])
+result_row_dtype = np.dtype([("grad_offset", np.int64), ("row", np.int32), ("n_sources", np.int32)])
 assert exposure_desc_dtype.itemsize == 32 and tile_dtype.itemsize == 40 and band_desc_dtype.itemsize == 24
 
 # every entry point of include/forcepho_b200.h with its ctypes signature
@@ -125,6 +126,8 @@ SIGNATURES = {
     "fp_hmc_lnprob": (ctypes.c_int, [c_vp, ctypes.c_int, c_vp, c_vp, c_vp, c_vp, ctypes.c_int, ctypes.c_int,
                                      c_vp, c_vp, c_vp]),
     "fp_hmc_leapfrog": (ctypes.c_int, [c_vp, ctypes.c_int, c_vp, ctypes.c_int, c_vp]),
+    "fp_upload_proposals": (ctypes.c_int, [c_vp, c_vp, ctypes.c_int, c_vp, c_vp]),
+    "fp_fetch_results": (ctypes.c_int, [c_vp, c_vp, c_vp, c_i64, c_vp, c_vp, c_vp]),
     "fp_measure_peaks": (ctypes.c_int, [c_vp, ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_double),
                                         c_vp]),
 }

@@ -20,7 +20,7 @@ import torch
 
 from . import _native as N
 from .autotune import Autotuner, size_class
-from .device import Plan, pack_proposals
+from .device import Plan, current_stream_ptr, pack_proposals, to_device_bytes
 from .kernel_limits import MAXBANDS, MAXSOURCES, NPARAMS
 from .structs import source_struct_dtype
 
@@ -64,24 +64,29 @@ class BatchedProposer:
 
         Proposals: the device layout, [n_patches][MAXSOURCES] records, written
         patch by patch as raw 264-byte records; a slot left over from a longer
-        earlier proposal is zeroed.  Results: only the (patch, band) rows that
-        exist are gathered on the device and copied back (chi2 and Response
-        records), in patch-major, band-minor order."""
+        earlier proposal is zeroed.  Only the records that a patch's kernels
+        read (its n_sources) go to the device.  Results: only the (patch, band)
+        rows that exist come back, in patch-major, band-minor order, each with
+        its n_sources x 7 derivatives."""
         dev = self.plan.device
         self._pin_prop = torch.zeros(self.plan.proposals.numel(), dtype=torch.uint8).pin_memory()
         self._prop_slots = self._pin_prop.numpy().view(_RECORD).reshape(self.n, MAXSOURCES)
         self._prop_len = [0] * self.n
         nb = [int(p.n_bands) for p in self.patches]
-        rows = [i * MAXBANDS + b for i in range(self.n) for b in range(nb[i])]
-        self._rows = torch.tensor(rows, dtype=torch.int64, device=dev)
-        self._dev_chi2 = torch.zeros(len(rows), dtype=torch.float64, device=dev)
-        self._dev_resp = torch.zeros((len(rows), MAXSOURCES * NPARAMS), dtype=torch.float32, device=dev)
-        self._pin_chi2 = torch.zeros(len(rows), dtype=torch.float64).pin_memory()
-        self._pin_resp = torch.zeros((len(rows), MAXSOURCES * NPARAMS), dtype=torch.float32).pin_memory()
-        offsets = np.concatenate([[0], np.cumsum(nb)[:-1]]).astype(int)
-        self._slices = [(slice(int(o), int(o) + nb[i]), (slice(int(o), int(o) + nb[i]),
-                                                         slice(0, int(self.patches[i].n_sources))))
-                        for i, o in enumerate(offsets)]
+        ns = [int(p.n_sources) for p in self.patches]
+        self._counts = torch.tensor(ns, dtype=torch.int32, device=dev)
+        rows = np.zeros(sum(nb), dtype=N.result_row_dtype)
+        self._slices = []
+        row = grad = 0
+        for i in range(self.n):
+            size = ns[i] * NPARAMS
+            self._slices.append((slice(row, row + nb[i]), slice(grad, grad + nb[i] * size), (nb[i], ns[i], NPARAMS)))
+            for b in range(nb[i]):
+                rows[row] = (grad, i * MAXBANDS + b, ns[i])
+                row, grad = row + 1, grad + size
+        self._rows = to_device_bytes(rows, dev)
+        self._pin_chi2 = torch.zeros(row, dtype=torch.float64).pin_memory()
+        self._pin_grad = torch.zeros(max(grad, 1), dtype=torch.float32).pin_memory()
         # completion of the last copy out of the proposal staging buffer and of
         # the last copy into the result buffers: the host waits on them before
         # rewriting the one or reading the others
@@ -157,8 +162,9 @@ class BatchedProposer:
             if k < lens[i]:
                 slots[i, k:lens[i]] = _ZERO_RECORD
             lens[i] = k
-        with torch.cuda.stream(s):
-            self.plan.proposals.copy_(self._pin_prop, non_blocking=True)
+        N.check(self.plan.L.fp_upload_proposals(self._pin_prop.data_ptr(), self._counts.data_ptr(), self.n,
+                                                self.plan.proposals.data_ptr(), current_stream_ptr(s)),
+                "fp_upload_proposals")
         self._h2d_done = torch.cuda.Event()
         self._h2d_done.record(s)
 
@@ -187,15 +193,12 @@ class BatchedProposer:
         return g
 
     def fetch_async(self, stream=None):
-        """Queue the device gather of the existing (patch, band) rows and their
-        copy into pinned host memory."""
+        """Queue the copy of the existing (patch, band) rows into pinned host memory."""
         s = stream or torch.cuda.current_stream()
-        with torch.cuda.stream(s):
-            torch.index_select(self.plan.chi2.view(-1), 0, self._rows, out=self._dev_chi2)
-            torch.index_select(self.plan.response.view(-1, MAXSOURCES * NPARAMS), 0, self._rows,
-                               out=self._dev_resp)
-            self._pin_chi2.copy_(self._dev_chi2, non_blocking=True)
-            self._pin_resp.copy_(self._dev_resp, non_blocking=True)
+        pl = self.plan
+        N.check(pl.L.fp_fetch_results(pl.chi2.data_ptr(), pl.response.data_ptr(), self._rows.data_ptr(),
+                                      self._pin_chi2.numel(), self._pin_chi2.data_ptr(), self._pin_grad.data_ptr(),
+                                      current_stream_ptr(s)), "fp_fetch_results")
         self._d2h_done = torch.cuda.Event()
         self._d2h_done.record(s)
 
@@ -206,8 +209,8 @@ class BatchedProposer:
         if self._d2h_done is not None:
             self._d2h_done.synchronize()
         c = self._pin_chi2.numpy().copy()
-        r = self._pin_resp.numpy().copy().reshape(-1, MAXSOURCES, NPARAMS)
-        return [(c[a], r[b]) for a, b in self._slices]
+        g = self._pin_grad.numpy().copy()
+        return [(c[a], g[b].reshape(shape)) for a, b, shape in self._slices]
 
     # --- the public call ---
     def evaluate_proposals(self, proposals, stream=None):
@@ -225,11 +228,11 @@ class BatchedProposer:
     # --- transfer accounting of one evaluate_proposals call ---
     @property
     def h2d_bytes(self):
-        return int(self.plan.proposals.numel())
+        return sum(int(p.n_sources) for p in self.patches) * source_struct_dtype.itemsize
 
     @property
     def d2h_bytes(self):
-        return int(self._pin_chi2.numel() * 8 + self._pin_resp.numel() * 4)
+        return int(self._pin_chi2.numel() * 8 + sum(b.stop - b.start for _, b, _ in self._slices) * 4)
 
     def count_pairs(self, stream=None):
         """(evaluated pairs, pairs within the cutoff, within-cutoff pairs culled) of one evaluation."""

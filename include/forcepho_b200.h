@@ -481,6 +481,27 @@ typedef struct fp_hmc_state {
 FP_API int fp_hmc_leapfrog(const fp_hmc_patch *d_hp, int n_patches, const fp_hmc_state *state, int stage,
                            void *stream);
 
+/* One (patch, band) row of a batch's results, for fp_fetch_results. */
+typedef struct fp_result_row {
+    int64_t grad_offset;    /* where its n_sources x NPARAMS derivatives go, in floats */
+    int32_t row;            /* patch * MAXBANDS + band: its chi2 and Response */
+    int32_t n_sources;
+} fp_result_row;
+
+/* Queue the copy of the first d_counts[p] source records of every patch p from
+ * h_records[p * MAXSOURCES ...] in page-locked host memory that the device can
+ * address to the same places of d_proposals.  The buffer must stay as it is
+ * until the copy has run.  No counterpart in the reference. */
+FP_API int fp_upload_proposals(const fp_source *h_records, const int32_t *d_counts, int n_patches,
+                               fp_source *d_proposals, void *stream);
+
+/* Queue the copy of n_rows rows of an evaluation's results into page-locked host
+ * memory that the device can address: h_chi2[i] and, at h_grad +
+ * d_rows[i].grad_offset, the derivatives of row i.  No counterpart in the
+ * reference. */
+FP_API int fp_fetch_results(const double *d_chi2, const fp_response *d_response, const fp_result_row *d_rows,
+                            int64_t n_rows, double *h_chi2, float *h_grad, void *stream);
+
 /* Size of the fixed device scratch array of fp_evaluate_batch_noalloc (32 MiB). */
 #define FP_NOALLOC_WORKSPACE_BYTES (32u << 20)
 
