@@ -19,8 +19,8 @@ backward, so both can be captured in a CUDA graph:
   derivatives from the device B-spline tables), then one batched evaluation
   (``fp_evaluate_batch``: Gaussian setup, the persistent tile kernel with its
   hand-written adjoint, the fixed-order reduction) gives chi2 and every
-  d chi2[band] / d(source parameter) in one pass; the Response records are
-  kept for backward;
+  d chi2[band] / d(source parameter) in one pass; those of the rows that
+  exist are kept for backward;
 * backward: the vector-Jacobian product with those per-band derivatives,
   assembled like ``stack_grad`` (forcepho/model.py:370-387) but kept per band,
   so any function of the band chi2s differentiates correctly: a band's flux
@@ -33,8 +33,8 @@ import numpy as np
 import torch
 
 from . import _native as N
-from .device import Plan, current_stream_ptr, to_device_bytes
-from .kernel_limits import MAXBANDS, MAXSOURCES, NPARAMS
+from .device import Plan, current_stream_ptr, result_rows, to_device_bytes
+from .kernel_limits import NPARAMS
 
 __all__ = ["BatchChi2", "PatchChi2"]
 
@@ -43,17 +43,17 @@ class _Chi2Fn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, theta, owner):
-        chi2, resp = owner._evaluate(theta.detach())
+        chi2, grads = owner._evaluate(theta.detach())
         ctx.owner = owner
         ctx.theta_meta = (theta.device, theta.dtype)
-        ctx.save_for_backward(resp)
+        ctx.save_for_backward(grads)
         return chi2
 
     @staticmethod
     def backward(ctx, grad_chi2):
-        (resp,) = ctx.saved_tensors
+        (grads,) = ctx.saved_tensors
         dev, dt = ctx.theta_meta
-        g = ctx.owner._vjp(grad_chi2.to(ctx.owner.device), resp)
+        g = ctx.owner._vjp(grad_chi2.to(ctx.owner.device), grads)
         return g.to(device=dev, dtype=dt), None
 
 
@@ -78,35 +78,24 @@ class BatchChi2(torch.nn.Module):
         dev = self.plan.device
         self.device = dev
         hp = np.zeros(self.n, dtype=N.hmc_patch_dtype)
-        rows, flux_idx, shape_idx = [], [], []
-        off = 0
+        first = np.zeros(self.n, dtype=np.int32)
+        off = nrow = 0
         self.slices, self.band_slices = [], []
-        nrow = 0
         for i, p in enumerate(self.patches):
             ns, nb = int(p.n_sources), int(p.n_bands)
             nper = nb + NPARAMS - 1
             hp[i] = (off, ns, nb)
+            first[i] = nrow
             self.slices.append(slice(off, off + ns * nper))
             self.band_slices.append(slice(nrow, nrow + nb))
-            rows += [i * MAXBANDS + b for b in range(nb)]
-            for s in range(ns):
-                for k in range(nper):
-                    j = off + s * nper + k
-                    if k < nb:      # flux in band k: Response[i, k, s, 0]
-                        flux_idx.append((j, ((i * MAXBANDS + k) * MAXSOURCES + s) * NPARAMS))
-                    else:           # shape parameter k - nb: column 1 + (k - nb) of every band
-                        shape_idx.append((j, (i * MAXSOURCES + s) * (NPARAMS - 1) + (k - nb)))
             off += ns * nper
             nrow += nb
         self.n_params = off
         self.n_rows = nrow
         self.d_hp = to_device_bytes(hp, dev)
-        i64 = dict(dtype=torch.int64, device=dev)
-        self._rows = torch.tensor(rows, **i64)
-        fi = np.array(flux_idx, np.int64).reshape(-1, 2)
-        si = np.array(shape_idx, np.int64).reshape(-1, 2)
-        self._flux_param, self._flux_src = torch.tensor(fi[:, 0], **i64), torch.tensor(fi[:, 1], **i64)
-        self._shape_param, self._shape_src = torch.tensor(si[:, 0], **i64), torch.tensor(si[:, 1], **i64)
+        self._h_rows, self._n_grads = result_rows(self.patches)
+        self._rows = to_device_bytes(self._h_rows, dev)
+        self._first_row = torch.from_numpy(first).to(dev)
         self._theta_buf = torch.zeros(max(off, 1), dtype=torch.float64, device=dev)
         self._jac_buf = torch.zeros(max(off, 1), dtype=torch.float64, device=dev)
         self.tab = spline_table(dev, splines)
@@ -114,33 +103,50 @@ class BatchChi2(torch.nn.Module):
 
     def _evaluate(self, theta):
         """Queue proposal construction and one evaluation at theta; returns
-        (chi2 rows, a copy of the Response records)."""
+        (chi2 rows, their derivatives), as ``fp_fetch_results`` lays them out."""
         if theta.shape != (self.n_params,):
             raise ValueError("theta has shape %s, expected (%d,)" % (tuple(theta.shape), self.n_params))
         th = theta.to(device=self.device, dtype=torch.float64).contiguous()
         s = current_stream_ptr()
+        pl = self.plan
         N.check(self.L.fp_hmc_prepare(self.d_hp.data_ptr(), self.n, th.data_ptr(), None, None,
-                                      ctypes.byref(self.tab), self.plan.proposals.data_ptr(),
+                                      ctypes.byref(self.tab), pl.proposals.data_ptr(),
                                       self._theta_buf.data_ptr(), self._jac_buf.data_ptr(), s), "fp_hmc_prepare")
-        self.plan.evaluate(self.launch)
+        pl.evaluate(self.launch)
         self.ncall += 1
-        chi2 = self.plan.chi2.view(-1).index_select(0, self._rows)
-        return chi2, self.plan.response.clone()
+        chi2 = torch.empty(self.n_rows, dtype=torch.float64, device=self.device)
+        grads = torch.empty(max(self._n_grads, 1), dtype=torch.float32, device=self.device)
+        N.check(self.L.fp_fetch_results(pl.chi2.data_ptr(), pl.response.data_ptr(), self._rows.data_ptr(),
+                                        self.n_rows, chi2.data_ptr(), grads.data_ptr(), s), "fp_fetch_results")
+        return chi2, grads
 
-    def _vjp(self, grad_chi2, resp):
-        """theta gradient of sum_rows grad_chi2[row] * chi2[row]."""
-        g2 = torch.zeros(self.n * MAXBANDS, dtype=torch.float64, device=self.device)
-        g2.index_copy_(0, self._rows, grad_chi2.to(torch.float64))
-        r = resp.view(self.n, MAXBANDS, MAXSOURCES, NPARAMS)
+    def _vjp(self, grad_chi2, grads):
+        """theta gradient of sum_rows grad_chi2[row] * chi2[row], in one launch
+        of 2 us (15 torch kernels over every slot took 40 us of the device and
+        bound small patches by their launches)."""
+        if torch.is_grad_enabled() and grad_chi2.requires_grad:
+            return self._vjp_differentiable(grad_chi2, grads)
+        g = grad_chi2.detach().to(torch.float64)
+        out = torch.empty(self.n_params, dtype=torch.float64, device=self.device)
+        N.check(self.L.fp_chi2_vjp(self.d_hp.data_ptr(), self.n, self._rows.data_ptr(), self._first_row.data_ptr(),
+                                   g.data_ptr(), g.stride(0), grads.data_ptr(), out.data_ptr(),
+                                   current_stream_ptr()), "fp_chi2_vjp")
+        return out
+
+    def _vjp_differentiable(self, grad_chi2, grads):
+        """The same product in torch operations, for a backward pass that is
+        itself differentiated by grad_chi2 (create_graph)."""
+        i64 = dict(dtype=torch.int64, device=self.device)
         out = torch.zeros(self.n_params, dtype=torch.float64, device=self.device)
-        # fluxes: one band each
-        fl = r.reshape(-1).index_select(0, self._flux_src).to(torch.float64)
-        out.index_copy_(0, self._flux_param, fl * g2.index_select(0, self._flux_src // (MAXSOURCES * NPARAMS)))
-        # shape parameters: summed over the bands with their weights
-        # (elementwise products and a sum: no library GEMM, so no handle or
-        # workspace to create inside a graph capture)
-        w = (g2.view(self.n, MAXBANDS, 1, 1) * r[..., 1:].to(torch.float64)).sum(dim=1)
-        out.index_copy_(0, self._shape_param, w.reshape(-1).index_select(0, self._shape_src))
+        for p, sl, rows in zip(self.patches, self.slices, self.band_slices):
+            ns, nb = int(p.n_sources), int(p.n_bands)
+            if ns == 0 or nb == 0:
+                continue
+            g0 = int(self._h_rows["grad_offset"][rows.start])
+            r = grads[g0:g0 + nb * ns * NPARAMS].view(nb, ns, NPARAMS).to(torch.float64)
+            g = grad_chi2[rows].to(torch.float64).view(nb, 1, 1)
+            whole = torch.cat([(g[..., 0] * r[..., 0]).T, (g * r[..., 1:]).sum(dim=0)], dim=1)
+            out = out.index_copy(0, torch.arange(sl.start, sl.stop, **i64), whole.reshape(-1))
         return out
 
     def forward(self, theta):

@@ -20,7 +20,7 @@ import torch
 
 from . import _native as N
 from .autotune import Autotuner, size_class
-from .device import Plan, current_stream_ptr, pack_proposals, to_device_bytes
+from .device import Plan, current_stream_ptr, pack_proposals, result_rows, to_device_bytes
 from .kernel_limits import MAXBANDS, MAXSOURCES, NPARAMS
 from .structs import source_struct_dtype
 
@@ -72,21 +72,17 @@ class BatchedProposer:
         self._pin_prop = torch.zeros(self.plan.proposals.numel(), dtype=torch.uint8).pin_memory()
         self._prop_slots = self._pin_prop.numpy().view(_RECORD).reshape(self.n, MAXSOURCES)
         self._prop_len = [0] * self.n
-        nb = [int(p.n_bands) for p in self.patches]
-        ns = [int(p.n_sources) for p in self.patches]
-        self._counts = torch.tensor(ns, dtype=torch.int32, device=dev)
-        rows = np.zeros(sum(nb), dtype=N.result_row_dtype)
-        self._slices = []
-        row = grad = 0
-        for i in range(self.n):
-            size = ns[i] * NPARAMS
-            self._slices.append((slice(row, row + nb[i]), slice(grad, grad + nb[i] * size), (nb[i], ns[i], NPARAMS)))
-            for b in range(nb[i]):
-                rows[row] = (grad, i * MAXBANDS + b, ns[i])
-                row, grad = row + 1, grad + size
+        self._counts = torch.tensor([int(p.n_sources) for p in self.patches], dtype=torch.int32, device=dev)
+        rows, n_grad = result_rows(self.patches)
+        self._slices, row, grad = [], 0, 0
+        for p in self.patches:
+            nb, ns = int(p.n_bands), int(p.n_sources)
+            size = nb * ns * NPARAMS
+            self._slices.append((slice(row, row + nb), slice(grad, grad + size), (nb, ns, NPARAMS)))
+            row, grad = row + nb, grad + size
         self._rows = to_device_bytes(rows, dev)
-        self._pin_chi2 = torch.zeros(row, dtype=torch.float64).pin_memory()
-        self._pin_grad = torch.zeros(max(grad, 1), dtype=torch.float32).pin_memory()
+        self._pin_chi2 = torch.zeros(len(rows), dtype=torch.float64).pin_memory()
+        self._pin_grad = torch.zeros(max(n_grad, 1), dtype=torch.float32).pin_memory()
         # completion of the last copy out of the proposal staging buffer and of
         # the last copy into the result buffers: the host waits on them before
         # rewriting the one or reading the others

@@ -21,39 +21,52 @@ namespace {
 constexpr int HMC_THREADS = 128;
 constexpr int MAXDEG = 5;
 
-// Nonzero B-spline basis functions of degree k at x, and their derivatives,
-// on the knot vector t of n coefficients (len(t) = n + k + 1).  x is clamped to
-// [t[k], t[n]] first, as FITPACK's bispev/parder do (so does scipy).
-// Cox-de Boor recurrence (de Boor, "A Practical Guide to Splines", ch. X);
-// returns the index of the first nonzero basis function.
-__device__ int bspline_basis(const double *__restrict__ t, int n, int k, double x, double *N, double *dN)
+// The span l of x in the knots t of n coefficients and degree k: t[l] <= x <
+// t[l+1], k <= l <= n-1, x == t[n] in the last one.  The lanes of `mask` compare
+// `width` knots at a time; `lane` counts them from 0.
+__device__ __forceinline__ int knot_span(const double *__restrict__ t, int n, int k, double x, unsigned mask, int lane,
+                                         int width)
 {
-    const double lo = t[k], hi = t[n];
-    x = fmin(fmax(x, lo), hi);
-    // span l: t[l] <= x < t[l+1], k <= l <= n-1 (x == hi falls in the last span)
-    int a = k, b = n - 1;
-    while (a < b) {
-        const int m = (a + b + 1) >> 1;
-        if (t[m] <= x) a = m; else b = m - 1;
+    int below = 0;
+    for (int i0 = 0; i0 <= n; i0 += width) {
+        const int i = i0 + lane;
+        below += __popc(__ballot_sync(mask, i <= n && t[i] <= x) & mask);
     }
-    const int l = a;
+    return max(k, min(n - 1, below - 1));
+}
+
+// Nonzero B-spline basis functions of degree k at x, and their derivatives, on
+// the knot vector t with x in span l.  Cox-de Boor recurrence (de Boor, "A
+// Practical Guide to Splines", ch. X).  DEG > 0: k = DEG is known, and the
+// arrays stay in registers.
+template <int DEG>
+__device__ __forceinline__ void bspline_basis(const double *__restrict__ t, int l, int deg, double x, double *N,
+                                              double *dN)
+{
+    const int k = DEG > 0 ? DEG : deg;
     double left[MAXDEG + 1], right[MAXDEG + 1], lower[MAXDEG + 1];
     N[0] = 1.0;
+#pragma unroll
     for (int j = 1; j <= k; ++j) {
         left[j] = x - t[l + 1 - j];
         right[j] = t[l + j] - x;
         double saved = 0.0;
+#pragma unroll
         for (int r = 0; r < j; ++r) {
             const double tmp = N[r] / (right[r + 1] + left[j - r]);
             N[r] = saved + right[r + 1] * tmp;
             saved = left[j - r] * tmp;
         }
         N[j] = saved;
-        if (j == k - 1)
+        if (j == k - 1) {
+#pragma unroll
             for (int r = 0; r <= j; ++r) lower[r] = N[r];
+        }
     }
+    if (k == 1) lower[0] = 1.0;
     // d/dx N_{i,k} = k (N_{i,k-1} / (t_{i+k} - t_i) - N_{i+1,k-1} / (t_{i+k+1} - t_{i+1}))
     // with N_{i,k-1} for i = l-k+1 .. l held in lower[0..k-1]
+#pragma unroll
     for (int r = 0; r <= k; ++r) {
         const int i = l - k + r;
         double d = 0.0;
@@ -67,74 +80,100 @@ __device__ int bspline_basis(const double *__restrict__ t, int n, int k, double 
         }
         dN[r] = k * d;
     }
-    return l - k;
 }
 
 __device__ __forceinline__ double sigm(double z) { return 1.0 / (1.0 + exp(-z)); }
 
 // --------------------------------------------------------------------------
-// transform + proposal: one thread per (patch, source)
+// transform + proposal: one warp per (patch, source)
 // --------------------------------------------------------------------------
-__global__ void __launch_bounds__(HMC_THREADS)
-prepare_kernel(const fp_hmc_patch *__restrict__ hp, int n_patches, const double *__restrict__ z,
-               const double *__restrict__ lower, const double *__restrict__ upper, fp_spline_table tab,
-               fp_source *__restrict__ props, double *__restrict__ theta, double *__restrict__ jac)
+// Latency bounds it: a thread per source ran the transforms, two knot searches,
+// the recurrences' divisions and 160 coefficient loads one after another, 20-24
+// us whatever the batch.  Here the lanes share the parameters, the knots (one
+// ballot per 16), the two axes (half a warp each) and the radii: 5.2 us for 12
+// sources, 5.5 us for 60.
+constexpr int PREPARE_WARPS = 2;
+
+template <int DEG>
+__global__ void __launch_bounds__(32 * PREPARE_WARPS)
+prepare_kernel(const fp_hmc_patch *__restrict__ hp, const double *__restrict__ z, const double *__restrict__ lower,
+               const double *__restrict__ upper, fp_spline_table tab, fp_source *__restrict__ props,
+               double *__restrict__ theta, double *__restrict__ jac)
 {
-    const int p = blockIdx.x;
+    const int p = blockIdx.x, lane = threadIdx.x & 31;
+    const int s = blockIdx.y * PREPARE_WARPS + (threadIdx.x >> 5);
     const fp_hmc_patch P = hp[p];
-    const int nper = P.n_bands + NPARAMS - 1;
-    for (int s = threadIdx.x; s < MAXSOURCES; s += blockDim.x) {
-        fp_source *src = props + (size_t)p * MAXSOURCES + s;
-        if (s >= P.n_sources) continue;
-        double th[MAXBANDS + NPARAMS - 1];
-        for (int k = 0; k < nper; ++k) {
-            const int64_t j = P.param_offset + (int64_t)s * nper + k;
-            const double zz = z[j];
-            double q = zz, J = 1.0;
-            if (lower != nullptr) {
-                const double rng = upper[j] - lower[j];
-                const double sg = sigm(zz);
-                q = lower[j] + rng * sg;
-                J = rng * sg * (1.0 - sg);
-            }
-            th[k] = q;
-            theta[j] = q;
-            jac[j] = J;
+    if (s >= P.n_sources) return;               // the whole warp
+    const int nb = P.n_bands, nper = nb + NPARAMS - 1;
+    const int64_t j0 = P.param_offset + (int64_t)s * nper;
+    fp_source *src = props + (size_t)p * MAXSOURCES + s;
+    const auto value = [&](int k, double *J) {
+        const double zz = z[j0 + k];
+        double q = zz;
+        *J = 1.0;
+        if (lower != nullptr) {
+            const double rng = upper[j0 + k] - lower[j0 + k];
+            const double sg = sigm(zz);
+            q = lower[j0 + k] + rng * sg;
+            *J = rng * sg * (1.0 - sg);
         }
-        const int nb = P.n_bands;
-        for (int b = 0; b < MAXBANDS; ++b) src->fluxes[b] = (b < nb) ? (float)th[b] : 0.f;
-        src->ra = (float)th[nb];
-        src->dec = (float)th[nb + 1];
-        src->q = (float)th[nb + 2];
-        src->pa = (float)th[nb + 3];
-        src->nsersic = (float)th[nb + 4];
-        src->rh = (float)th[nb + 5];
-        // A_r(sersic, rhalf) and its partial derivatives from the tensor-product spline
-        double Nx[MAXDEG + 1], dNx[MAXDEG + 1], Ny[MAXDEG + 1], dNy[MAXDEG + 1];
-        const int ncx = tab.nx - tab.kx - 1, ncy = tab.ny - tab.ky - 1;
-        const int ix = bspline_basis(tab.tx, ncx, tab.kx, th[nb + 4], Nx, dNx);
-        const int iy = bspline_basis(tab.ty, ncy, tab.ky, th[nb + 5], Ny, dNy);
-        for (int r = 0; r < MAXRADII; ++r) {
-            double a = 0.0, an = 0.0, ar = 0.0;
-            if (r < tab.n_radii) {
-                const double *c = tab.coef + (size_t)r * ncx * ncy;
-                for (int u = 0; u <= tab.kx; ++u) {
-                    const double *row = c + (size_t)(ix + u) * ncy + iy;
-                    double sv = 0.0, sd = 0.0;
-                    for (int v = 0; v <= tab.ky; ++v) {
-                        sv += row[v] * Ny[v];
-                        sd += row[v] * dNy[v];
-                    }
-                    a += Nx[u] * sv;
-                    an += dNx[u] * sv;
-                    ar += Nx[u] * sd;
-                }
+        return q;
+    };
+    for (int k = lane; k < nper; k += 32) {
+        double J;
+        const double q = value(k, &J);
+        theta[j0 + k] = q;
+        jac[j0 + k] = J;
+        if (k < nb) src->fluxes[k] = (float)q;
+        else (&src->ra)[k - nb] = (float)q;     // ra, dec, q, pa, nsersic, rh
+    }
+    for (int b = nb + lane; b < MAXBANDS; b += 32) src->fluxes[b] = 0.f;
+
+    // A_r(sersic, rhalf) and its partial derivatives from the tensor-product
+    // spline: the lower half of the warp forms the basis in sersic, the upper
+    // half in rhalf.  x is clamped to the knots' range first, as FITPACK's
+    // bispev/parder do (so does scipy).
+    const int half = lane >> 4;
+    const int ncx = tab.nx - tab.kx - 1, ncy = tab.ny - tab.ky - 1;
+    const double *t = half ? tab.ty : tab.tx;
+    const int n = half ? ncy : ncx, k = half ? tab.ky : tab.kx;
+    double J, N[MAXDEG + 1], dN[MAXDEG + 1];
+    const double x = fmin(fmax(value(nb + 4 + half, &J), t[k]), t[n]);
+    const int l = knot_span(t, n, k, x, half ? 0xffff0000u : 0x0000ffffu, lane & 15, 16);
+    bspline_basis<DEG>(t, l, k, x, N, dN);
+    const int ix = __shfl_sync(0xffffffffu, l, 0) - tab.kx, iy = __shfl_sync(0xffffffffu, l, 16) - tab.ky;
+    constexpr int TOP = DEG > 0 ? DEG : MAXDEG;
+    double Nx[TOP + 1], dNx[TOP + 1], Ny[TOP + 1], dNy[TOP + 1];
+#pragma unroll
+    for (int u = 0; u <= TOP; ++u) {
+        Nx[u] = __shfl_sync(0xffffffffu, N[u], 0);
+        dNx[u] = __shfl_sync(0xffffffffu, dN[u], 0);
+        Ny[u] = __shfl_sync(0xffffffffu, N[u], 16);
+        dNy[u] = __shfl_sync(0xffffffffu, dN[u], 16);
+    }
+    if (lane >= MAXRADII) return;
+    double a = 0.0, an = 0.0, ar = 0.0;
+    if (lane < tab.n_radii) {
+        const double *c = tab.coef + (size_t)lane * ncx * ncy;
+#pragma unroll
+        for (int u = 0; u <= TOP; ++u) {
+            if (DEG == 0 && u > tab.kx) break;
+            const double *row = c + (size_t)(ix + u) * ncy + iy;
+            double sv = 0.0, sd = 0.0;
+#pragma unroll
+            for (int v = 0; v <= TOP; ++v) {
+                if (DEG == 0 && v > tab.ky) break;
+                sv += row[v] * Ny[v];
+                sd += row[v] * dNy[v];
             }
-            src->mixture_amplitudes[r] = (float)a;
-            src->damplitude_dnsersic[r] = (float)an;
-            src->damplitude_drh[r] = (float)ar;
+            a += Nx[u] * sv;
+            an += dNx[u] * sv;
+            ar += Nx[u] * sd;
         }
     }
+    src->mixture_amplitudes[lane] = (float)a;
+    src->damplitude_dnsersic[lane] = (float)an;
+    src->damplitude_drh[lane] = (float)ar;
 }
 
 // --------------------------------------------------------------------------
@@ -187,6 +226,31 @@ lnprob_kernel(const fp_hmc_patch *__restrict__ hp, const double *__restrict__ z,
         double c = 0.0;
         for (int b = 0; b < nb; ++b) c += chi2[(size_t)p * MAXBANDS + b];
         lnp[p] = -0.5 * c + lj;
+    }
+}
+
+// --------------------------------------------------------------------------
+// vector-Jacobian product of the band chi2s: one CTA per patch
+// --------------------------------------------------------------------------
+// out[theta] = sum over bands of g[row] dchi2[row]/dtheta, from the rows that
+// fetch_kernel copied: a flux moves its own band, a shape parameter every band.
+__global__ void __launch_bounds__(HMC_THREADS)
+vjp_kernel(const fp_hmc_patch *__restrict__ hp, const fp_result_row *__restrict__ rows,
+           const int32_t *__restrict__ first_row, const double *__restrict__ g, int64_t g_stride,
+           const float *__restrict__ grads, double *__restrict__ out)
+{
+    const int p = blockIdx.x;
+    const fp_hmc_patch P = hp[p];
+    const int nb = P.n_bands, nper = nb + NPARAMS - 1;
+    const int64_t r0 = first_row[p];
+    for (int j = threadIdx.x; j < P.n_sources * nper; j += blockDim.x) {
+        const int s = j / nper, k = j - s * nper;
+        const int b0 = k < nb ? k : 0, b1 = k < nb ? k + 1 : nb;
+        const int col = s * NPARAMS + (k < nb ? 0 : 1 + (k - nb));
+        double acc = 0.0;
+        for (int b = b0; b < b1; ++b)
+            acc += g[(r0 + b) * g_stride] * (double)grads[rows[r0 + b].grad_offset + col];
+        out[P.param_offset + j] = acc;
     }
 }
 
@@ -295,8 +359,13 @@ extern "C" int fp_hmc_prepare(const fp_hmc_patch *d_hp, int n_patches, const dou
         tab->ky > MAXDEG || tab->nx < 2 * tab->kx + 2 || tab->ny < 2 * tab->ky + 2 || !tab->tx || !tab->ty ||
         !tab->coef)
         return fp_set_error(FP_ERR_ARGUMENT, "fp_hmc_prepare: bad spline table");
-    prepare_kernel<<<n_patches, 32, 0, (cudaStream_t)stream>>>(d_hp, n_patches, d_z, d_lower, d_upper, *tab,
-                                                               d_proposals, d_theta, d_jac);
+    const dim3 blocks((unsigned)n_patches, (MAXSOURCES + PREPARE_WARPS - 1) / PREPARE_WARPS);
+    if (tab->kx == 3 && tab->ky == 3)           // the bicubic splines of the amplitude table
+        prepare_kernel<3><<<blocks, 32 * PREPARE_WARPS, 0, (cudaStream_t)stream>>>(d_hp, d_z, d_lower, d_upper, *tab,
+                                                                                   d_proposals, d_theta, d_jac);
+    else
+        prepare_kernel<0><<<blocks, 32 * PREPARE_WARPS, 0, (cudaStream_t)stream>>>(d_hp, d_z, d_lower, d_upper, *tab,
+                                                                                   d_proposals, d_theta, d_jac);
     return fp_check_cuda(cudaGetLastError(), "prepare_kernel launch");
 }
 
@@ -309,6 +378,17 @@ extern "C" int fp_hmc_lnprob(const fp_hmc_patch *d_hp, int n_patches, const doub
     lnprob_kernel<<<n_patches, HMC_THREADS, 0, (cudaStream_t)stream>>>(d_hp, d_z, d_jac, d_chi2, d_response,
                                                                        transformed, sampling, d_lnp, d_grad);
     return fp_check_cuda(cudaGetLastError(), "lnprob_kernel launch");
+}
+
+extern "C" int fp_chi2_vjp(const fp_hmc_patch *d_hp, int n_patches, const fp_result_row *d_rows,
+                           const int32_t *d_first_row, const double *d_g, int64_t g_stride, const float *d_grads,
+                           double *d_out, void *stream)
+{
+    if (!d_hp || n_patches < 1 || !d_rows || !d_first_row || !d_g || g_stride < 0 || !d_grads || !d_out)
+        return fp_set_error(FP_ERR_ARGUMENT, "fp_chi2_vjp: bad arguments");
+    vjp_kernel<<<n_patches, HMC_THREADS, 0, (cudaStream_t)stream>>>(d_hp, d_rows, d_first_row, d_g, g_stride, d_grads,
+                                                                    d_out);
+    return fp_check_cuda(cudaGetLastError(), "vjp_kernel launch");
 }
 
 extern "C" int fp_hmc_leapfrog(const fp_hmc_patch *d_hp, int n_patches, const fp_hmc_state *state, int stage,

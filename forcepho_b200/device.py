@@ -323,6 +323,21 @@ def pack_proposals(proposals, n_patches):
     return out
 
 
+def result_rows(patches):
+    """``fp_result_row`` records of every (patch, band) of a plan, patch-major
+    and band-minor, their derivatives one after another; and how many floats
+    those are."""
+    nb = np.array([int(p.n_bands) for p in patches], np.int64)
+    ns = np.array([int(p.n_sources) for p in patches], np.int64)
+    rows = np.zeros(int(nb.sum()), dtype=N.result_row_dtype)
+    band = np.arange(len(rows)) - np.repeat(np.cumsum(nb) - nb, nb)
+    rows["row"] = np.repeat(np.arange(len(nb)), nb) * MAXBANDS + band
+    rows["n_sources"] = np.repeat(ns, nb)
+    size = np.repeat(ns, nb) * NPARAMS
+    rows["grad_offset"] = np.cumsum(size) - size
+    return rows, int(size.sum())
+
+
 def response_view(resp_host, n_bands, n_sources):
     """(n_bands, n_sources, NPARAMS) float32 view of Response records, as the
     reference reshapes them (forcepho/proposal.py:139-141)."""

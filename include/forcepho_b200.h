@@ -496,11 +496,20 @@ FP_API int fp_upload_proposals(const fp_source *h_records, const int32_t *d_coun
                                fp_source *d_proposals, void *stream);
 
 /* Queue the copy of n_rows rows of an evaluation's results into page-locked host
- * memory that the device can address: h_chi2[i] and, at h_grad +
+ * memory that the device can address, or device memory: h_chi2[i] and, at h_grad +
  * d_rows[i].grad_offset, the derivatives of row i.  No counterpart in the
  * reference. */
 FP_API int fp_fetch_results(const double *d_chi2, const fp_response *d_response, const fp_result_row *d_rows,
                             int64_t n_rows, double *h_chi2, float *h_grad, void *stream);
+
+/* Queue d_out[j] = sum over rows of d_g[row * g_stride] * dchi2[row]/dtheta_j for
+ * every scene parameter of every patch (d_hp's layout): the vector-Jacobian
+ * product of the band chi2s.  d_grads holds the derivatives as fp_fetch_results
+ * lays them out (device memory here), d_rows its rows, d_first_row[p] the first
+ * of patch p's n_bands rows.  No counterpart in the reference. */
+FP_API int fp_chi2_vjp(const fp_hmc_patch *d_hp, int n_patches, const fp_result_row *d_rows,
+                       const int32_t *d_first_row, const double *d_g, int64_t g_stride, const float *d_grads,
+                       double *d_out, void *stream);
 
 /* Size of the fixed device scratch array of fp_evaluate_batch_noalloc (32 MiB). */
 #define FP_NOALLOC_WORKSPACE_BYTES (32u << 20)
