@@ -12,7 +12,11 @@
 //     (band_start/N, n_psf_per_source, exposure_start/N) back to the host (two
 //     waits on the stream) and compares them, and the xpix/ypix pointers, with
 //     the cached plan's; any difference makes a new plan from the device
-//     coordinates (one more read-back);
+//     coordinates (one more read-back).  The read-backs land in page-locked
+//     memory: six copies into pageable memory wait for the stream one by one
+//     (126 us a call on a patch of 8 sources and 8 exposures, 96 us
+//     now).  The arrays are read at the addresses of the struct just read,
+//     never of the cached one: those may have been freed since;
 //   * the tile bounding boxes are recomputed on the device at every call, so a
 //     plan stays exact even when the coordinates are rewritten in place at the
 //     same addresses (the pixel order then only loses compactness);
@@ -21,6 +25,8 @@
 //
 // Calls on one patch must not overlap on the GPU (they share its workspace),
 // which the reference's synchronous pycuda call never does either.
+
+#include <string.h>
 
 #include <algorithm>
 #include <mutex>
@@ -49,6 +55,28 @@ struct ref_plan {
 std::mutex g_mu;
 std::vector<ref_plan> g_plans;
 unsigned long long g_clock = 0;
+
+// Page-locked landing place of the read-backs, used under g_mu and kept until
+// fp_evaluate_proposal_release(); grown to the largest patch's index arrays.
+unsigned char *g_pinned = nullptr;
+size_t g_pinned_bytes = 0;
+
+int pinned(size_t bytes, unsigned char **out)
+{
+    if (bytes > g_pinned_bytes) {
+        if (g_pinned) cudaFreeHost(g_pinned);
+        g_pinned = nullptr;
+        g_pinned_bytes = 0;
+        void *p = nullptr;
+        const size_t n = bytes < 4096 ? 4096 : bytes;
+        if (int rc = fp_check_cuda(cudaHostAlloc(&p, n, cudaHostAllocPortable), "fp_evaluate_proposal: host buffer"))
+            return rc;
+        g_pinned = static_cast<unsigned char *>(p);
+        g_pinned_bytes = n;
+    }
+    *out = g_pinned;
+    return FP_OK;
+}
 constexpr size_t MAX_PLANS = 64;
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -191,35 +219,57 @@ extern "C" int fp_evaluate_proposal(const fp_patch *d_patch, const fp_source *d_
     int dev = 0;
     if (int rc = fp_check_cuda(cudaGetDevice(&dev), "cudaGetDevice")) return rc;
 
-    // 1. the struct
-    fp_patch hp;
-    if (int rc = fp_check_cuda(cudaMemcpyAsync(&hp, d_patch, sizeof(fp_patch), cudaMemcpyDeviceToHost, st),
-                               "fp_evaluate_proposal: read patch struct"))
-        return rc;
-    if (int rc = fp_check_cuda(cudaStreamSynchronize(st), "fp_evaluate_proposal: stream")) return rc;
-    if (hp.n_sources != n_sources)
-        return fp_set_error(FP_ERR_ARGUMENT, "fp_evaluate_proposal: n_sources=%d but the patch has %d", n_sources,
-                            hp.n_sources);
-
     std::lock_guard<std::mutex> lock(g_mu);
     ref_plan *hit = nullptr;
     for (ref_plan &p : g_plans)
         if (p.device == dev && p.d_patch == d_patch) hit = &p;
+
+    // 1. the struct
+    const size_t nb = (size_t)n_bands;
+    unsigned char *host = nullptr;
+    if (int rc = pinned(sizeof(fp_patch), &host)) return rc;
+    if (int rc = fp_check_cuda(cudaMemcpyAsync(host, d_patch, sizeof(fp_patch), cudaMemcpyDeviceToHost, st),
+                               "fp_evaluate_proposal: read patch struct"))
+        return rc;
+    if (int rc = fp_check_cuda(cudaStreamSynchronize(st), "fp_evaluate_proposal: stream")) return rc;
+    fp_patch hp;
+    memcpy(&hp, host, sizeof(hp));
+    if (hp.n_sources != n_sources)
+        return fp_set_error(FP_ERR_ARGUMENT, "fp_evaluate_proposal: n_sources=%d but the patch has %d", n_sources,
+                            hp.n_sources);
 
     // 2. the index arrays (the exposure arrays sized from band_N, known from
     // the cached plan when the layout has not changed)
     ref_plan cur;
     cur.device = dev;
     cur.d_patch = d_patch;
-    if (int rc = read_back(cur.band_start, hp.band_start, (size_t)n_bands, st, "band_start")) return rc;
-    if (int rc = read_back(cur.band_N, hp.band_N, (size_t)n_bands, st, "band_N")) return rc;
-    if (int rc = read_back(cur.n_psf, hp.n_psf_per_source, (size_t)n_bands, st, "n_psf_per_source")) return rc;
-    size_t n_exp_guess = (hit && same_layout(hit->key, hp)) ? hit->exposure_start.size() : 0;
-    if (n_exp_guess) {
-        if (int rc = read_back(cur.exposure_start, hp.exposure_start, n_exp_guess, st, "exposure_start")) return rc;
-        if (int rc = read_back(cur.exposure_N, hp.exposure_N, n_exp_guess, st, "exposure_N")) return rc;
-    }
-    if (int rc = fp_check_cuda(cudaStreamSynchronize(st), "fp_evaluate_proposal: read index arrays")) return rc;
+    const size_t n_exp_guess = (hit && same_layout(hit->key, hp)) ? hit->exposure_start.size() : 0;
+    const size_t o_bn = align256(nb * sizeof(int16_t)), o_psf = 2 * o_bn, o_es = align256(o_psf + nb * sizeof(int32_t));
+    const size_t o_en = align256(o_es + n_exp_guess * sizeof(int32_t));
+    if (int rc = pinned(o_en + n_exp_guess * sizeof(int32_t), &host)) return rc;
+    const auto ask = [&](size_t o, const void *src, size_t n, const char *what) {
+        if (n == 0) return (int)FP_OK;
+        if (!src) return fp_set_error(FP_ERR_ARGUMENT, "fp_evaluate_proposal: patch without %s", what);
+        return fp_check_cuda(cudaMemcpyAsync(host + o, src, n, cudaMemcpyDeviceToHost, st), what);
+    };
+    int asked = ask(0, hp.band_start, nb * sizeof(int16_t), "band_start");
+    if (asked == FP_OK) asked = ask(o_bn, hp.band_N, nb * sizeof(int16_t), "band_N");
+    if (asked == FP_OK) asked = ask(o_psf, hp.n_psf_per_source, nb * sizeof(int32_t), "n_psf_per_source");
+    if (asked == FP_OK) asked = ask(o_es, hp.exposure_start, n_exp_guess * sizeof(int32_t), "exposure_start");
+    if (asked == FP_OK) asked = ask(o_en, hp.exposure_N, n_exp_guess * sizeof(int32_t), "exposure_N");
+    // also after a refused copy: those before it must not land in a later call's buffer
+    const cudaError_t waited = cudaStreamSynchronize(st);
+    if (asked != FP_OK) return asked;
+    if (int rc = fp_check_cuda(waited, "fp_evaluate_proposal: read index arrays")) return rc;
+    const auto take = [&](auto &dst, size_t o, size_t n) {
+        dst.resize(n);
+        if (n) memcpy(dst.data(), host + o, n * sizeof(dst[0]));
+    };
+    take(cur.band_start, 0, nb);
+    take(cur.band_N, o_bn, nb);
+    take(cur.n_psf, o_psf, nb);
+    take(cur.exposure_start, o_es, n_exp_guess);
+    take(cur.exposure_N, o_en, n_exp_guess);
     int64_t n_exp = 0;
     for (int b = 0; b < n_bands; ++b) {
         if (cur.band_N[b] < 0 || cur.band_start[b] != n_exp)
@@ -268,5 +318,8 @@ extern "C" int fp_evaluate_proposal_release(void)
     std::lock_guard<std::mutex> lock(g_mu);
     for (ref_plan &p : g_plans) free_plan(p);
     g_plans.clear();
+    if (g_pinned) cudaFreeHost(g_pinned);
+    g_pinned = nullptr;
+    g_pinned_bytes = 0;
     return FP_OK;
 }
