@@ -300,6 +300,39 @@ __device__ __forceinline__ void stage(const staged_gauss &s, int i, const float4
     s.g2[i] = {fp_dup(B.y), make_float2(A.y, B.x)};
 }
 
+// Whether the region {E = dx^T F dx <= MAX_EXP_ARG (1% margin)} of a Gaussian
+// (FP32 pixel-loop parameters A = (xc, yc, c Fxx, c Fxy), fys = c Fyy) meets
+// the rectangle [x0,x1] x [y0,y1]: the minimum of the convex quadratic over the
+// rectangle is at the centre if it lies inside, else on an edge, where it is a
+// clamped 1-D minimum.  FP32: near the threshold the centre lies within the
+// Gaussian's cutoff radius of the rectangle, so the offsets x0 - cx, ... are
+// exact wherever the coordinates exceed that radius (Sterbenz: within a factor
+// 2 of each other); where they do not, the coordinates are small and an offset
+// error d moves E by only about 12 d / sigma.  The quadratic form's rounding
+// error (~1e-4 of E) is far inside the 1% margin (0.36) as well.  No
+// Gaussian with a pixel of the rectangle within the cutoff is dropped; the
+// pair census checks exactly that.  Non-finite results keep the Gaussian.
+__device__ __forceinline__ bool ellipse_meets_rect(const float4 A, float fys, float x0, float x1, float y0,
+                                                   float y1)
+{
+    const float ic = (float)(1.0 / FP_EXP2_SCALE);
+    const float cx = A.x, cy = A.y, fxx = A.z * ic, fxy = A.w * ic, fyy = fys * ic;
+    if (cx >= x0 && cx <= x1 && cy >= y0 && cy <= y1) return true;
+    const float rxx = __frcp_rn(fxx), ryy = __frcp_rn(fyy);
+    float best = INFINITY;
+    const float lx = x0 - cx, hx = x1 - cx, ly = y0 - cy, hy = y1 - cy;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const float dx = k ? hx : lx;
+        const float dy = fminf(fmaxf(-fxy * dx * ryy, ly), hy);
+        best = fminf(best, fmaf(fxx * dx, dx, fmaf(2.f * fxy * dx, dy, fyy * dy * dy)));
+        const float ey = k ? hy : ly;
+        const float ex = fminf(fmaxf(-fxy * ey * rxx, lx), hx);
+        best = fminf(best, fmaf(fxx * ex, ex, fmaf(2.f * fxy * ex, ey, fyy * ey * ey)));
+    }
+    return !(best > (float)(MAX_EXP_ARG * 1.01));
+}
+
 // How a warp's pixels meet a Gaussian.  ROWS: every thread's 4 pixels lie in
 // one row, so the y terms are formed once per thread.  Otherwise they are
 // formed per pixel, with F dx's second component as c Fyy dy + fma'd c Fxy dx
@@ -310,14 +343,16 @@ __device__ __forceinline__ void stage(const staged_gauss &s, int i, const float4
 enum forward_form { ROWS, SAME_Y, ANY_Y, MIXED };
 
 // Adds the run's Gaussians in `word` (bit i: s.g*[r0 + i]) to 4 pixels' FP32
-// sums, in ascending order.
+// sums, in ascending order.  Nine in ten bits are set, so four at a time are
+// mostly due: their loads and exponentials then overlap and one test serves
+// them (forward-only tile kernel of 48 field patches 1.83 ms one by one, 1.72
+// two, 1.65 four, 1.67 eight at a time; testing each Gaussian's ellipse against
+// the warp's pixels, or 16x8 pixel warps with a tighter box, gained nothing).
 template <forward_form FORM>
 __device__ __forceinline__ void forward_run(unsigned word, int r0, const staged_gauss &s, const fp_f2 (&x)[2],
                                             const fp_f2 (&y)[2], bool same_y, float (&m)[4], float (&mc)[4])
 {
-#pragma unroll 1
-    for (int i = r0; word != 0u; ++i, word >>= 1) {
-        if ((word & 1u) == 0u) continue;
+    const auto visit = [&](int i) {
         const fp_f4 g0 = s.g0[i], g1 = s.g1[i], g2 = s.g2[i];
         const float yc = g2.y.x, fyy = g2.y.y;
         const float dy0 = y[0].x - yc;
@@ -345,6 +380,20 @@ __device__ __forceinline__ void forward_run(unsigned word, int r0, const staged_
             m[2 * k] = (e.x < FP_CUT_SCALED) ? m[2 * k] : fmaf(ga, h.x, m[2 * k]);
             m[2 * k + 1] = (e.y < FP_CUT_SCALED) ? m[2 * k + 1] : fmaf(gb, h.y, m[2 * k + 1]);
 #endif
+        }
+    };
+    int i = r0;
+#pragma unroll 1
+    while (word != 0u) {
+        if (FORM != MIXED && (word & 15u) == 15u) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) visit(i + u);
+            i += 4;
+            word >>= 4;
+        } else {
+            if (word & 1u) visit(i);
+            ++i;
+            word >>= 1;
         }
     }
 }
@@ -875,39 +924,6 @@ __device__ __forceinline__ void grid_partials(const float4 A, float Fyy, const d
     S[5] += -H11 + (b * ((double)m[2][0] + m[0][2]) + t * m[1][1]) * (1.0 / 12.0);
 }
 #endif
-
-// Whether the region {E = dx^T F dx <= MAX_EXP_ARG (1% margin)} of a Gaussian
-// (FP32 pixel-loop parameters A = (xc, yc, c Fxx, c Fxy), fys = c Fyy) meets
-// the rectangle [x0,x1] x [y0,y1]: the minimum of the convex quadratic over the
-// rectangle is at the centre if it lies inside, else on an edge, where it is a
-// clamped 1-D minimum.  FP32: near the threshold the centre lies within the
-// Gaussian's cutoff radius of the rectangle, so the offsets x0 - cx, ... are
-// exact wherever the coordinates exceed that radius (Sterbenz: within a factor
-// 2 of each other); where they do not, the coordinates are small and an offset
-// error d moves E by only about 12 d / sigma.  The quadratic form's rounding
-// error (~1e-4 of E) is far inside the 1% margin (0.36) as well.  No
-// Gaussian with a pixel of the rectangle within the cutoff is dropped; the
-// pair census checks exactly that.  Non-finite results keep the Gaussian.
-__device__ __forceinline__ bool ellipse_meets_rect(const float4 A, float fys, float x0, float x1, float y0,
-                                                   float y1)
-{
-    const float ic = (float)(1.0 / FP_EXP2_SCALE);
-    const float cx = A.x, cy = A.y, fxx = A.z * ic, fxy = A.w * ic, fyy = fys * ic;
-    if (cx >= x0 && cx <= x1 && cy >= y0 && cy <= y1) return true;
-    const float rxx = __frcp_rn(fxx), ryy = __frcp_rn(fyy);
-    float best = INFINITY;
-    const float lx = x0 - cx, hx = x1 - cx, ly = y0 - cy, hy = y1 - cy;
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const float dx = k ? hx : lx;
-        const float dy = fminf(fmaxf(-fxy * dx * ryy, ly), hy);
-        best = fminf(best, fmaf(fxx * dx, dx, fmaf(2.f * fxy * dx, dy, fyy * dy * dy)));
-        const float ey = k ? hy : ly;
-        const float ex = fminf(fmaxf(-fxy * ey * rxx, lx), hx);
-        best = fminf(best, fmaf(fxx * ex, ex, fmaf(2.f * fxy * ex, ey, fyy * ey * ey)));
-    }
-    return !(best > (float)(MAX_EXP_ARG * 1.01));
-}
 
 struct tile_smem {
     size_t g, box, pix, wsrc, red, ints, rows, keepw, idx, total;
