@@ -843,26 +843,24 @@ __device__ __forceinline__ void partials_to_grad(const double *__restrict__ J, i
 //     dx^i once at the strip's end, stand for all 15;
 //   * the exponent is dx^2 Fxx + dy (2 Fxy dx + Fyy dy), two operations with
 //     the column's products formed beforehand.
-// That leaves 9 operations per pixel, paired over columns (packed FP32) where
-// that costs no more of the register ports than scalar ones (a packed
-// multiply-add of three different pairs takes 3 cycles, two scalar ones that
-// share the row's dy take 2), and 2 per row of 4 pixels.  Four columns are what
-// 64 registers hold (10 sums each pair).  Sums run over at most 32 rows in
-// FP32, as the list's do; the step from the 15 sums to the image-space partials
-// is FP64.  Sums about the strip's centre instead, with constant weights, ran
-// 5 % faster but cost Gaussians narrower than the strip two decimal digits when
-// shifted; 16 rows a sum cost 3 % and gained no digit.
+// That leaves 9 operations per pixel, paired over columns (packed FP32), and
+// 2 per row of 4 pixels.  Four columns are what 64 registers hold (10 sums
+// each pair).  Sums run over at most 32 rows in FP32, as the list's do; the
+// step from the 15 sums to the image-space partials is FP64.  Sums about the
+// strip's centre instead, with constant weights, ran 5 % faster but cost
+// Gaussians narrower than the strip two decimal digits when shifted.
 // Tile kernel on 48 field patches (2.9e9 evaluated pairs): 6.31 ms with the
-// list, 3.72 ms with this and the forward pass as it is now (1.64 ms of it); on
-// a 30-source patch of 32 exposures of 256x256 px, 1.64 and 0.91 ms.
-__device__ __forceinline__ void grid_partials(const float4 A, float Fyy, const float *__restrict__ s_w, int r,
-                                              int rend, int step, float x, float y0, double (&S)[6])
+// list, 4.02 ms here; on a 30-source patch of 32 exposures of 256x256 px,
+// 1.64 and 0.98 ms.
+__device__ __forceinline__ void grid_partials(const float4 A, float Fyy, const double *__restrict__ J,
+                                              int64_t n_gauss, const float *__restrict__ s_w, int r, int rend, int step, float x,
+                                              float y0, double (&S)[6])
 {
     float dx[4], m[5][5];
 #pragma unroll
     for (int k = 0; k < 4; ++k) dx[k] = (x + (float)k) - A.x;
     {
-        const fp_f2 nyc = fp_dup(-A.y), ystep = fp_dup((float)step);
+        const fp_f2 nyc = fp_dup(-A.y), fyy = fp_dup(Fyy), ystep = fp_dup((float)step);
         fp_f2 y = fp_dup(y0 + (float)r);
         fp_f2 l[2], q[2], Y[5][2];
 #pragma unroll
@@ -880,51 +878,35 @@ __device__ __forceinline__ void grid_partials(const float4 A, float Fyy, const f
             const fp_f2 dy = __fadd2_rn(y, nyc);
             y = __fadd2_rn(y, ystep);
             const fp_f2 yy = __fmul2_rn(dy, dy);
-            fp_f2 e[2], K[2], t[2];
-#pragma unroll
-            for (int k = 0; k < 2; ++k) e[k] = make_float2(fmaf(dy.x, Fyy, l[k].x), fmaf(dy.x, Fyy, l[k].y));
-#pragma unroll
-            for (int k = 0; k < 2; ++k) e[k] = make_float2(fmaf(dy.x, e[k].x, q[k].x), fmaf(dy.x, e[k].y, q[k].y));
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
-                // past the cutoff 2^-200 is an exact zero (ex2 flushes it, and the
-                // grid holds finite weights only)
-                e[k].x = (e[k].x < FP_CUT_SCALED) ? -200.f : e[k].x;
-                e[k].y = (e[k].y < FP_CUT_SCALED) ? -200.f : e[k].y;
-                K[k] = __fmul2_rn(k ? w.y : w.x, make_float2(fp_ex2(e[k].x), fp_ex2(e[k].y)));
+                const fp_f2 e = __ffma2_rn(dy, __ffma2_rn(fyy, dy, l[k]), q[k]);
+                const fp_f2 g = __fmul2_rn(k ? w.y : w.x, make_float2(fp_ex2(e.x), fp_ex2(e.y)));
+                const fp_f2 K = make_float2((e.x < FP_CUT_SCALED) ? 0.f : g.x, (e.y < FP_CUT_SCALED) ? 0.f : g.y);
+                Y[0][k] = __fadd2_rn(Y[0][k], K);
+                Y[1][k] = __ffma2_rn(K, dy, Y[1][k]);
+                const fp_f2 t = __fmul2_rn(K, yy);
+                Y[2][k] = __fadd2_rn(Y[2][k], t);
+                Y[3][k] = __ffma2_rn(t, dy, Y[3][k]);
+                Y[4][k] = __ffma2_rn(t, yy, Y[4][k]);
             }
-#pragma unroll
-            for (int k = 0; k < 2; ++k) t[k] = __fmul2_rn(K[k], yy);
-#pragma unroll
-            for (int k = 0; k < 2; ++k) Y[0][k] = __fadd2_rn(Y[0][k], K[k]);
-#pragma unroll
-            for (int k = 0; k < 2; ++k) Y[1][k] = __ffma2_rn(K[k], dy, Y[1][k]);
-#pragma unroll
-            for (int k = 0; k < 2; ++k) Y[2][k] = __fadd2_rn(Y[2][k], t[k]);
-#pragma unroll
-            for (int k = 0; k < 2; ++k) Y[3][k] = __ffma2_rn(t[k], dy, Y[3][k]);
-#pragma unroll
-            for (int k = 0; k < 2; ++k) Y[4][k] = __ffma2_rn(t[k], yy, Y[4][k]);
         }
         // m[i][j] = sum K dx^i dy^j over the strip
-        const fp_f2 dxa = make_float2(dx[0], dx[1]), dxb = make_float2(dx[2], dx[3]);
 #pragma unroll
         for (int j = 0; j < 5; ++j) {
-            fp_f2 ya = Y[j][0], yb = Y[j][1];
+            const float t[4] = {Y[j][0].x, Y[j][0].y, Y[j][1].x, Y[j][1].y};
+            m[0][j] = (t[0] + t[1]) + (t[2] + t[3]);
+            float p[4] = {t[0], t[1], t[2], t[3]};
 #pragma unroll
-            for (int i = 0; i < 5 - j; ++i) {
-                if (i > 0) {
-                    ya = __fmul2_rn(ya, dxa);
-                    yb = __fmul2_rn(yb, dxb);
-                }
-                const fp_f2 sum = __fadd2_rn(ya, yb);
-                m[i][j] = sum.x + sum.y;
+            for (int i = 1; i < 5 - j; ++i) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) p[k] *= dx[k];
+                m[i][j] = (p[0] + p[1]) + (p[2] + p[3]);
             }
         }
     }
     // H = h + |F dx|^2 / 24, h = 1 - tr F / 24
-    const double ic = 1.0 / FP_EXP2_SCALE;
-    const double a = ic * A.z, b = ic * A.w, c = ic * Fyy;
+    const double a = J[n_gauss], b = J[2 * n_gauss], c = J[3 * n_gauss];
     const double t = a + c;
     const double xx = a * a + b * b, xy = b * t, yy = b * b + c * c;      // F^2
     const double h = 1.0 - t * (1.0 / 24.0);
@@ -1169,9 +1151,9 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
                         first += n;
                         if (b0 >= b1) continue;
                         const int rend = lo + min(nrow, b1 * kr);
-                        grid_partials(A, fyy, reinterpret_cast<const float *>(s_pix) + 4 * j,
-                                      valid ? lo + b0 * kr + rep : rend, rend, kr, grid.x0 + (float)(4 * j), grid.y0,
-                                      S);
+                        grid_partials(A, fyy, J, n_gauss, reinterpret_cast<const float *>(s_pix) + 4 * j,
+                                      valid ? lo + b0 * kr + rep : rend, rend, kr, grid.x0 + (float)(4 * j),
+                                      grid.y0, S);
                     }
                 } else
 #endif
