@@ -34,7 +34,8 @@ import numpy as np
 import torch
 
 from . import _native as N
-from .device import Plan, pack_proposals, to_device_bytes
+from .device import PackedArrays, Plan, pack_proposals
+from .sources import pack_proposal
 from .structs import patch_struct_dtype, ptr_dtype, source_struct_dtype
 
 __all__ = ["SceneView", "subtract_fixed", "design_models", "design_matrix", "normal_equations", "render"]
@@ -50,31 +51,47 @@ class SceneView:
     ``residual`` are device addresses chosen by the caller (e.g. an all-zero
     array and an output row, so the residual is minus the scene's model)."""
 
-    def __init__(self, parent, scene, data_ptr, residual_ptr):
+    def __init__(self, parent, scene, data_ptr, residual_ptr, meta=None, packed=None):
         if getattr(parent, "device_patch", None) is None:
             raise ValueError("the parent patch must be sent to the device first")
         self.parent = parent
         for name in ("exposure_start", "exposure_N", "band_start", "band_N", "n_psf_per_source",
                      "xpix", "ypix"):
             setattr(self, name, getattr(parent, name))
-        meta = parent.meta_for(scene)
+        meta = parent.meta_for(scene) if meta is None else meta
         self.n_sources = int(meta["n_sources"])
-        dev = parent._dev()
-        self._keep = {k: to_device_bytes(np.ascontiguousarray(meta[k]), dev) for k in _VIEW_META}
+        # the metadata and the struct reach the device in one copy: this view's
+        # own, or one for several views (``scene_views``)
+        own = packed is None
+        packed = PackedArrays() if own else packed
+        self._packed = packed
+        self._ptrs = (int(data_ptr), int(residual_ptr))
+        self._arrays = {k: np.ascontiguousarray(meta[k]) for k in _VIEW_META}
+        self._at = {k: packed.place_once(a) for k, a in self._arrays.items()}
+        self._at["struct"] = packed.place(patch_struct_dtype.itemsize)
+        if own:
+            packed.allocate()
+            self._fill(packed.reserve(parent._dev()))
+            packed.copy()
+
+    def _fill(self, base):
+        """Write the arrays and the struct (with the device addresses from
+        ``base`` on) into the packed host buffer."""
+        parent, packed = self.parent, self._packed
         s = np.zeros(1, dtype=patch_struct_dtype)
         for name in patch_struct_dtype.names:
             if patch_struct_dtype[name] == ptr_dtype:
-                if name in self._keep:
-                    s[name] = int(self._keep[name].data_ptr())
+                if name in self._arrays:
+                    s[name] = base + self._at[name]
                 elif name in parent.device_ptrs:
                     s[name] = parent.device_ptrs[name].ptr
             else:
                 s[name] = getattr(parent, name)
         s["n_sources"] = self.n_sources
-        s["data"] = int(data_ptr)
-        s["residual"] = int(residual_ptr)
-        self.device_patch = torch.empty(patch_struct_dtype.itemsize, dtype=torch.uint8, device=dev)
-        self.device_patch.copy_(torch.from_numpy(s.view(np.uint8).copy()))
+        s["data"], s["residual"] = self._ptrs
+        o, n = self._at["struct"], patch_struct_dtype.itemsize
+        packed.host[o:o + n] = s.view(np.uint8)
+        self.device_patch = packed.device[o:o + n]
 
     @property
     def npix(self):
@@ -91,6 +108,20 @@ class SceneView:
     @property
     def device_patch_ptr(self):
         return int(self.device_patch.data_ptr())
+
+
+def scene_views(parent, scenes, data_ptrs, residual_ptrs):
+    """A SceneView of each scene; all their metadata in one copy to the device."""
+    packed = PackedArrays()
+    metas = parent.metas_for(scenes) if hasattr(parent, "metas_for") else [parent.meta_for(sc) for sc in scenes]
+    views = [SceneView(parent, sc, d, r, meta=m, packed=packed)
+             for sc, d, r, m in zip(scenes, data_ptrs, residual_ptrs, metas)]
+    packed.allocate()
+    base = packed.reserve(parent._dev())
+    for v in views:
+        v._fill(base)
+    packed.copy()
+    return views
 
 
 def _tile_pixels(patch):
@@ -110,30 +141,31 @@ def _forward_only(views, proposals, ctas_per_sm=4):
     return plan
 
 
-def _scene_view(patch, scene, data_ptr, residual_ptr):
-    """A SceneView of ``scene`` (from ``patch.set_scene``) and the scene, with
-    its positions as the offsets the metadata and proposals take.  A
-    store-backed patch's ``set_scene`` gives absolute positions (its
-    ``pack_meta`` zeroes them): the scene is zeroed at its own median, as the
-    reference's ``pack_meta`` does for every scene it renders, and the patch's
-    own reference coordinate is left as it was.  A synthetic patch's catalog
-    already holds offsets."""
+def _scene_views(patch, scenes, data_ptrs, residual_ptrs):
+    """SceneViews of ``scenes`` (from ``patch.set_scene``), with their positions
+    as the offsets the metadata and proposals take.  A store-backed patch's
+    ``set_scene`` gives absolute positions (its ``pack_meta`` zeroes them): each
+    scene is zeroed at its own median, as the reference's ``pack_meta`` does for
+    every scene it renders, and the patch's own reference coordinate is left as
+    it was.  A synthetic patch's catalog already holds offsets."""
     if not hasattr(patch, "zerocoords"):
-        return SceneView(patch, scene, data_ptr, residual_ptr), scene
+        return scene_views(patch, scenes, data_ptrs, residual_ptrs)
     saved = np.array(patch.patch_reference_coordinates, dtype=np.float64, copy=True)
+    views = []
     try:
-        patch.zerocoords(scene)
-        view = SceneView(patch, scene, data_ptr, residual_ptr)
+        for scene, d, r in zip(scenes, data_ptrs, residual_ptrs):
+            patch.zerocoords(scene)
+            views.append(SceneView(patch, scene, d, r))
     finally:
         patch.patch_reference_coordinates = saved
-    return view, scene
+    return views
 
 
 def _scene_proposal(scene):
     srcs = list(scene.sources)
     if not srcs:
         return np.zeros(0, dtype=source_struct_dtype)
-    return np.concatenate([s.proposal().copy() for s in srcs])
+    return pack_proposal(srcs)
 
 
 def _blocks(catalog, maxactive):
@@ -192,12 +224,10 @@ def design_models(patch, active):
         return X[:, :patch.npix], scene
     zeros = torch.zeros(max(patch.npix, 1), dtype=torch.float32, device=dev)
     from .sources import Scene
-    views, props = [], []
-    for i, g in enumerate(scene.sources):
-        v, one = _scene_view(patch, Scene([copy.copy(g)]), zeros.data_ptr(), X[i].data_ptr())
-        views.append(v)
-        props.append(_scene_proposal(one))
-    plan = _forward_only(views, props)
+    ones = [Scene([copy.copy(g)]) for g in scene.sources]
+    views = _scene_views(patch, ones, [zeros.data_ptr()] * n, [X[i].data_ptr() for i in range(n)])
+    props = _scene_proposal(Scene([one.sources[0] for one in ones]))
+    plan = _forward_only(views, [props[i:i + 1] for i in range(n)])
     X.neg_()                                             # residual of zero data = -model
     flux = torch.tensor(np.array([g.flux for g in scene.sources], dtype=np.float64),
                         dtype=torch.float32, device=dev)
@@ -251,7 +281,7 @@ def render(patch, catalog, splinedata=None, unpack=True):
     npix = max(patch.npix, 1)
     zeros = torch.zeros(npix, dtype=torch.float32, device=dev)
     out = torch.empty(npix, dtype=torch.float32, device=dev)
-    view, scene = _scene_view(patch, scene, zeros.data_ptr(), out.data_ptr())
+    (view,) = _scene_views(patch, [scene], [zeros.data_ptr()], [out.data_ptr()])
     plan = _forward_only([view], [_scene_proposal(scene)])
     del plan, view
     model = (-out[:patch.npix]).cpu().numpy()

@@ -67,6 +67,15 @@ class SersicSplines:
     def damplitude_drh(self, sersic, rhalf):
         return np.array([float(s(sersic, rhalf, dy=1)[0, 0]) for s in self.splines])
 
+    def evaluate(self, sersic, rhalf):
+        """``(amplitudes, damplitude_dsersic, damplitude_drh)``, each
+        [n_sources, n_radii], at the points (sersic[i], rhalf[i]): the values of
+        the three methods above, bit for bit, with one call per radius for all
+        sources instead of one per radius and source."""
+        x, y = np.atleast_1d(np.asarray(sersic, np.float64)), np.atleast_1d(np.asarray(rhalf, np.float64))
+        return tuple(np.stack([s.ev(x, y, **kw) for s in self.splines], axis=1)
+                     for kw in ({}, {"dx": 1}, {"dy": 1}))
+
     def tck(self):
         """Knots and coefficients of every spline: (tx, ty, c[n_radii, ...], kx, ky).
 

@@ -74,29 +74,41 @@ class SyntheticPatch(B200PatchMixin, PatchBase):
         srcs = list(scene.sources)
         ns, ne = len(srcs), self.n_exp
         dt = self.meta_dtype
+        ra = np.array([g.ra for g in srcs], np.float64)
+        dec = np.array([g.dec for g in srcs], np.float64)
+        cosd = np.cos(np.deg2rad(REF_COORD[1] + dec))
         D = np.zeros((ne, ns, 2, 2), dtype=dt)
         CW = np.zeros((ne, ns, 2, 2), dtype=dt)
         crpix = np.zeros((ne, ns, 2), dtype=dt)
         crval = np.zeros((ne, ns, 2), dtype=dt)
-        for e in range(ne):
-            for s, g in enumerate(srcs):
-                cosd = np.cos(np.deg2rad(REF_COORD[1] + g.dec))
-                W = np.diag([cosd, 1.0])
-                D[e, s] = A[e]
-                CW[e, s] = 3600.0 * A[e] @ W
-                crval[e, s] = [g.ra, g.dec]
-                crpix[e, s] = cen[e] + A[e] @ (3600.0 * W @ np.array([g.ra, g.dec]))
+        D[:] = A[:, None]
+        A3600 = 3600.0 * A[:, None]
+        CW[..., 0] = A3600[..., 0] * cosd[:, None]
+        CW[..., 1] = A3600[..., 1]
+        crval[..., 0], crval[..., 1] = ra, dec
+        # tangent-plane offsets in arcsec
+        u, v = (3600.0 * cosd) * ra, 3600.0 * dec
+        crpix[:] = cen[:, None] + (A[:, None, :, 0] * u[:, None] + A[:, None, :, 1] * v[:, None])
         # every source of an exposure gets a copy of the exposure's PSF block
-        blocks, pstart, k = [], [], 0
-        for e in range(ne):
-            one = self.psf_blocks[e]
-            pstart.append(k)
-            for _ in range(ns):
-                blocks.append(one)
-                k += len(one)
-        psfgauss = np.concatenate(blocks) if blocks else np.zeros(0, psf_dtype)
+        sizes = np.array([len(b) for b in self.psf_blocks], np.int64) * ns
+        pstart = np.cumsum(sizes) - sizes
+        psfgauss = (np.concatenate([np.tile(b, ns) for b in self.psf_blocks]) if ne and ns
+                    else np.zeros(0, psf_dtype))
         return dict(n_sources=ns, D=D, CW=CW, crpix=crpix, crval=crval, psfgauss=psfgauss,
                     psfgauss_start=np.asarray(pstart, dtype=np.int32))
+
+    def metas_for(self, scenes):
+        """``meta_for`` of each of several scenes.  Scenes of one source each are
+        cut out of one evaluation; their PSF records, the same for every source,
+        are one array."""
+        scenes = list(scenes)
+        if (len(scenes) < 2 or any(len(sc.sources) != 1 for sc in scenes)
+                or type(self).meta_for is not SyntheticPatch.meta_for):
+            return [self.meta_for(sc) for sc in scenes]
+        whole = self.meta_for(Scene([sc.sources[0] for sc in scenes]))
+        first = self.meta_for(scenes[0])
+        return [dict(first, **{k: whole[k][:, i:i + 1] for k in ("D", "CW", "crpix", "crval")})
+                for i in range(len(scenes))]
 
     def pack_meta(self, scene):
         """Make ``scene`` the patch's scene: repack its source metadata
