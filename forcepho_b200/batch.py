@@ -11,8 +11,9 @@ three launches of one evaluation are captured once into a CUDA graph and
 replayed.
 
 ``evaluate_proposals(list of source_struct arrays)`` is the public call:
-host proposals -> pinned staging -> device, graph replay, chi2 and Response
-records back to the host, returned per patch in the reference's shapes.
+host proposals -> pinned staging -> device, graph replay, the existing rows of
+chi2 and derivatives back to the host, returned per patch in the reference's
+shapes.
 """
 
 import numpy as np

@@ -14,7 +14,7 @@
 //                  do not lose the precision of large pixel coordinates.
 //                  Per tile:
 //                  1. cull: keep the Gaussians whose box, and then whose
-//                     E <= MAX_EXP_ARG ellipse (FP64), meets the tile's pixel
+//                     E <= MAX_EXP_ARG ellipse, meets the tile's pixel
 //                     box; every other Gaussian has E > MAX_EXP_ARG at every
 //                     pixel of the tile and contributes exactly nothing;
 //                  2. forward, pixel-parallel: 4 pixels per thread, Gaussians
@@ -419,7 +419,8 @@ __device__ __forceinline__ void forward_run(unsigned word, int r0, const staged_
 // bound the loop, which any mix of packed and scalar operations runs within 2 %.
 // Forward-only tile kernel with one pixel per thread in 256-pixel tiles, all
 // scalar, and as here: 58 and 46 us on a 16-source patch of 10 exposures of
-// 150x150 px (256-pixel tiles), 2.00 and 1.82 ms on 48 field patches.
+// 150x150 px (256-pixel tiles), 2.00 and 1.82 ms on 48 field patches (1.65
+// with forward_run's four Gaussians at a time).
 // s_m: 1024 doubles for those sums, free until the adjoint.
 template <int P>
 __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure_desc &ed, const fp_patch *pt,
@@ -849,9 +850,10 @@ __device__ __forceinline__ void partials_to_grad(const double *__restrict__ J, i
 // step from the 15 sums to the image-space partials is FP64.  Sums about the
 // strip's centre instead, with constant weights, ran 5 % faster but cost
 // Gaussians narrower than the strip two decimal digits when shifted.
-// Tile kernel on 48 field patches (2.9e9 evaluated pairs): 6.31 ms with the
-// list, 4.02 ms here; on a 30-source patch of 32 exposures of 256x256 px,
-// 1.64 and 0.98 ms.
+// Tile kernel on 48 field patches (2.9e9 evaluated pairs): 6.19 ms with the
+// list, 3.77 ms here; on a 30-source patch of 32 exposures of 256x256 px,
+// 1.64 and 0.92 ms; on a 16-source patch of 10 exposures of 150x150 px
+// (256-pixel tiles), 120 and 88 us.
 __device__ __forceinline__ void grid_partials(const float4 A, float Fyy, const double *__restrict__ J,
                                               int64_t n_gauss, const float *__restrict__ s_w, int r, int rend, int step, float x,
                                               float y0, double (&S)[6])

@@ -204,7 +204,7 @@ FP_API int fp_evaluate_proposal_f64(const fp_patch *d_patch, const fp_source *d_
  * coordinates), then queues three launches that produce the results
  * asynchronously on `stream`.  Tile bounding boxes are recomputed every call,
  * so coordinates rewritten in place stay exact.  Plans (tables and workspace:
- * about 216 B per image Gaussian plus 40 B per pixel tile) are device memory
+ * about 208 B per image Gaussian plus 40 B per pixel tile) are device memory
  * owned by the library, at most 64 of them (least recently used first out),
  * until fp_evaluate_proposal_release.  Calls on one patch must not overlap on
  * the GPU: they share its plan's workspace.  n_sources must equal the struct's
