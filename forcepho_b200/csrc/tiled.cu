@@ -32,7 +32,8 @@
 //                     chunk's last, partial group of v Gaussians is
 //                     replicated over the idle lanes, each replica taking
 //                     every k-th row or pixel, and the replicas summed by
-//                     shuffles).  Power sums of the offsets give the 6
+//                     shuffles).  Power sums of the offsets (across
+//                     and along the Gaussian's ridge) give the 6
 //                     image-space partials, which the FP64 Jacobian maps to
 //                     the 7 on-sky partials once per (Gaussian, segment), not
 //                     once per pixel;
@@ -266,6 +267,7 @@ struct tile_grid {
     int strip[8];
 };
 constexpr int FP_GRID_STRIDE = 36;      // floats per row: 8 replicas' rows start in different banks
+constexpr float FP_GRID_WEIGHT_MAX = 0x1p60f;   // larger weights could leave FP32 in the grid's fourth powers
 
 // Whether a tile's box allows the grid: its pixels lie within the cell of its
 // class, which the planner's compact tiles do, and the box starts at integers.
@@ -289,6 +291,7 @@ struct staged_gauss {
     fp_f4 *g0;      // (-xc, -xc), (c Fxx, c Fxx)
     fp_f4 *g1;      // (c Fxy, c Fxy), (A C24, A C24)
     fp_f4 *g2;      // (A k0, A k0), (yc, c Fyy)
+    fp_f2 *ridge;   // (Fxy / Fyy, c (Fxx - Fxy^2 / Fyy)), for the adjoint over the weight grid
 };
 
 __device__ __forceinline__ void stage(const staged_gauss &s, int i, const float4 *__restrict__ gfwd,
@@ -298,6 +301,32 @@ __device__ __forceinline__ void stage(const staged_gauss &s, int i, const float4
     s.g0[i] = {fp_dup(-A.x), fp_dup(A.z)};
     s.g1[i] = {fp_dup(A.w), fp_dup(B.z)};
     s.g2[i] = {fp_dup(B.y), make_float2(A.y, B.x)};
+}
+
+// The ridge of staged Gaussian i.  s is the quotient of the FP32 values; the
+// exponent's coefficient of dx^2 follows from it in FP64 (J: the Gaussian's
+// Jacobian terms), where the two sides would cancel in FP32.
+__device__ __forceinline__ void stage_ridge(const staged_gauss &sg, int i, const double *__restrict__ J,
+                                            int64_t n_gauss)
+{
+    const float slope = sg.g1[i].x.x / sg.g2[i].y.y;
+    const double a = J[n_gauss], b = J[2 * n_gauss], c = J[3 * n_gauss], s = slope;
+    sg.ridge[i] = make_float2(slope, (float)(FP_EXP2_SCALE * (a - s * b - s * (b - s * c))));
+}
+
+// Whether the adjoint over the weight grid may take staged Gaussian i with this
+// box.  The box is finite only where F is positive definite: the exponent is
+// then negative everywhere, also where the tile has no weight.  The other
+// bounds (widths of 2^-12 to 2^12 pixels, a centre within 2^20, a ridge not
+// steeper than 2^10) keep every product of the ridge coordinates finite: |dx|
+// < 2^21, |u| < 2^32, and |u| < 2^15 wherever K > 0.  Any other Gaussian sends
+// its tile to the pixel list.
+__device__ __forceinline__ bool gauss_suits_grid(const staged_gauss &s, int i, const float4 box)
+{
+    const float fxx = s.g0[i].y.x, fyy = s.g2[i].y.y;       // times c < 0
+    return isfinite(box.x) && isfinite(box.y) && isfinite(box.z) && isfinite(box.w) && fxx < -0x1p-24f &&
+           fxx > -0x1p24f && fyy < -0x1p-24f && fyy > -0x1p24f && fabsf(s.g1[i].x.x) <= -0x1p10f * fyy &&
+           fabsf(s.g0[i].x.x) <= 0x1p20f && fabsf(s.g2[i].y.x) <= 0x1p20f;
 }
 
 // Whether the region {E = dx^T F dx <= MAX_EXP_ARG (1% margin)} of a Gaussian
@@ -426,8 +455,8 @@ template <int P>
 __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure_desc &ed, const fp_patch *pt,
                                             const int32_t *__restrict__ perm, const float4 *__restrict__ pix,
                                             const float4 *__restrict__ gfwd, const float4 *__restrict__ gbox,
-                                            const float2 *__restrict__ gctr, const float ox, const float oy,
-                                            const bool nocull, const int gc, const uint16_t *s_idx,
+                                            const float2 *__restrict__ gctr, const double *__restrict__ gjac,
+                                            const int64_t n_gauss, const float ox, const float oy, const bool nocull, const int gc, const uint16_t *s_idx,
                                             const staged_gauss &sg, float4 *s_gbox, float4 *s_pix, int *s_int,
                                             double *s_red, double *s_m, unsigned *s_rows, tile_grid &grid)
 {
@@ -466,6 +495,7 @@ __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure
     };
     if (P < 4) load();
 
+    bool fits = grid.on;        // what this thread has seen of the tile suits the weight grid
     // warps per set of the tile's pixels, and the sets; each set takes every
     // sets-th run of Gaussians
     const int per_set = npix > 512 ? 8 : npix > 256 ? 4 : npix > 128 ? 2 : 1;
@@ -538,7 +568,12 @@ __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure
             for (int i = tid; i < cn; i += FP_THREADS) {
                 const int64_t gi = ed.gauss_offset + s_idx[c0 + i];
                 stage(sg, i, gfwd, gctr, gi, ox, oy);
-                s_gbox[i] = gbox[gi];
+                const float4 box = gbox[gi];
+                s_gbox[i] = box;
+                if (grid.on) {
+                    stage_ridge(sg, i, gjac + gi, n_gauss);
+                    fits = fits && gauss_suits_grid(sg, i, box);
+                }
             }
             __syncthreads();
             // runs of 32 Gaussians: lane l tests Gaussian r0 + l against the
@@ -634,14 +669,13 @@ __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure
     for (int o = 16; o > 0; o >>= 1) chi += __shfl_down_sync(0xffffffffu, chi, o);
     if (lane == 31) s_int[8 + warp] = incl;
     if (lane == 0) s_red[warp] = chi;
-    bool fits = grid.on;
     if (grid.on) {
         if (gc == 0) __syncthreads();       // no pass over Gaussians ordered the clearing above
 #pragma unroll
         for (int k = 0; k < P; ++k)
             if (ws[k] != 0.f) {
                 const float gx = xs[k] - grid.x0, gy = ys[k] - grid.y0;
-                const bool in = isfinite(ws[k]) && gx >= 0.f && gx < (float)grid.cols && gy >= 0.f &&
+                const bool in = fabsf(ws[k]) <= FP_GRID_WEIGHT_MAX && gx >= 0.f && gx < (float)grid.cols && gy >= 0.f &&
                                 gy < (float)grid.rows && gx == truncf(gx) && gy == truncf(gy);
                 fits = fits && in;
                 if (in) atomicOr(&s_rows[(int)gy], 1u << (int)gx);
@@ -837,38 +871,58 @@ __device__ __forceinline__ void partials_to_grad(const double *__restrict__ J, i
 //
 // FP32 operations bound the adjoint.  The list takes 30 per pixel: the
 // offsets, the exponent, H and 12 sums, all about the Gaussian's own centre.
-// Here
-//   * H is a quadratic form of the offsets, so every moment of K and KH is a
-//     combination of the 15 sums of K dx^i dy^j, i + j <= 4;
-//   * down a column dx is fixed: 5 sums of K dy^j per column, weighted with
-//     dx^i once at the strip's end, stand for all 15;
-//   * the exponent is dx^2 Fxx + dy (2 Fxy dx + Fyy dy), two operations with
-//     the column's products formed beforehand.
-// That leaves 9 operations per pixel, paired over columns (packed FP32), and
-// 2 per row of 4 pixels.  Four columns are what 64 registers hold (10 sums
-// each pair).  Sums run over at most 32 rows in FP32, as the list's do; the
-// step from the 15 sums to the image-space partials is FP64.  Sums about the
-// strip's centre instead, with constant weights, ran 5 % faster but cost
-// Gaussians narrower than the strip two decimal digits when shifted.
+// Here dx is fixed down a column, and the row offset is taken from the
+// Gaussian's ridge, u = dy + s dx with s = Fxy / Fyy:
+//   * E = P dx^2 + Fyy u^2, P = Fxx - Fxy^2 / Fyy: one operation per pixel on
+//     the u^2 that the sums need anyway;
+//   * H and the offsets are polynomials in (dx, u), so the 15 sums of
+//     K dx^i u^j, i + j <= 4, give every moment, and per column the 5 sums of
+//     K u^j, weighted with dx^i once at the strip's end, give those.
+// That leaves 10 operations per pixel, paired over columns (packed FP32), and
+// one per row of 4 pixels.  Four columns are what 64 registers hold (10 sums
+// each pair).
 // Tile kernel on 48 field patches (2.9e9 evaluated pairs): 6.19 ms with the
-// list, 3.77 ms here; on a 30-source patch of 32 exposures of 256x256 px,
-// 1.64 and 0.92 ms; on a 16-source patch of 10 exposures of 150x150 px
-// (256-pixel tiles), 120 and 88 us.
-__device__ __forceinline__ void grid_partials(const float4 A, float Fyy, const double *__restrict__ J,
-                                              int64_t n_gauss, const float *__restrict__ s_w, int r, int rend, int step, float x,
+// list, 3.77 ms with FP32 sums of plain dy^j, 3.86 ms here; on a 30-source
+// patch of 32 exposures of 256x256 px, 1.64, 0.92 and 0.94 ms; on a 16-source
+// patch of 10 exposures of 150x150 px (256-pixel tiles), 120, 88 and 91 us.
+// The FP64 column sums are 1.5 % of the field patches' time.
+//
+// Precision.  Sums of plain dy^j would cancel in E, H and F wherever the
+// Gaussian is thin and oblique; dx and u are the axes in which E has no mixed
+// term.  Any s will do as long as the same one is used throughout: the FP32
+// quotient is, and what it misses of Fxy / Fyy enters the FP64 step.  A column's
+// ridge is held relative to the integer row nearest the strip's, so that its
+// rounding is that of a few pixels, not of the tile's extent.  A column's FP32
+// sum runs over at most 32 pixels, as the list's do, and is FP64 from there on.
+// Largest error of a gradient column against 64 bits on three faint sources
+// with white-noise weights, 12 draws (list; plain dy^j; here): q 0.1 7e-5,
+// 9e-3, 2e-6; q 0.2 1.1e-5, 3.6e-4, 1.6e-6; q 0.35 1.5e-6, 4.4e-6, 4e-7; q 0.6
+// 5e-7, 4e-7, 3e-7; q 0.9 7e-7, 6e-7, 6e-7.
+//
+// Range.  gauss_suits_grid admits the Gaussians and forward_tile the weights
+// (FP_GRID_WEIGHT_MAX) for which no product and no sum of 32 rows leaves FP32,
+// at places without a weight (0 times a finite number) as elsewhere.
+//
+// Adds the strip's sums to S in ridge coordinates: KH, then the gradient by
+// (dx, u) and by the coefficients of (dx^2, u^2, 2 dx u), all but the first as
+// ridge_to_partials takes them.  ridge: the staged pair; fyy: c Fyy.
+__device__ __forceinline__ void grid_partials(const float xc, const float yc, const float fyy, const fp_f2 ridge,
+                                              const double *__restrict__ J, int64_t n_gauss,
+                                              const float *__restrict__ s_w, int r, int rend, int step, float x,
                                               float y0, double (&S)[6])
 {
-    float dx[4], m[5][5];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) dx[k] = (x + (float)k) - A.x;
+    fp_f2 Y[5][2];
     {
-        const fp_f2 nyc = fp_dup(-A.y), fyy = fp_dup(Fyy), ystep = fp_dup((float)step);
-        fp_f2 y = fp_dup(y0 + (float)r);
-        fp_f2 l[2], q[2], Y[5][2];
+        // the integer row nearest the ridge in the strip's middle
+        const float row = rintf(fmaf(-ridge.x, (x + 1.5f) - xc, yc)), yr = yc - row;
+        const fp_f2 ystep = fp_dup((float)step), f = fp_dup(fyy);
+        fp_f2 y = fp_dup((y0 + (float)r) - row);
+        fp_f2 c[2], q[2];
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-            l[k] = make_float2((2.f * A.w) * dx[2 * k], (2.f * A.w) * dx[2 * k + 1]);
-            q[k] = make_float2((A.z * dx[2 * k]) * dx[2 * k], (A.z * dx[2 * k + 1]) * dx[2 * k + 1]);
+            const float da = (x + (float)(2 * k)) - xc, db = (x + (float)(2 * k + 1)) - xc;
+            c[k] = make_float2(fmaf(ridge.x, da, -yr), fmaf(ridge.x, db, -yr));
+            q[k] = make_float2((ridge.y * da) * da, (ridge.y * db) * db);
 #pragma unroll
             for (int j = 0; j < 5; ++j) Y[j][k] = fp_dup(0.f);
         }
@@ -877,58 +931,76 @@ __device__ __forceinline__ void grid_partials(const float4 A, float Fyy, const d
 #pragma unroll 1
         for (; pw < pend; pw += step * FP_GRID_STRIDE) {
             const fp_f4 w = *reinterpret_cast<const fp_f4 *>(pw);
-            const fp_f2 dy = __fadd2_rn(y, nyc);
-            y = __fadd2_rn(y, ystep);
-            const fp_f2 yy = __fmul2_rn(dy, dy);
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
-                const fp_f2 e = __ffma2_rn(dy, __ffma2_rn(fyy, dy, l[k]), q[k]);
-                const fp_f2 g = __fmul2_rn(k ? w.y : w.x, make_float2(fp_ex2(e.x), fp_ex2(e.y)));
-                const fp_f2 K = make_float2((e.x < FP_CUT_SCALED) ? 0.f : g.x, (e.y < FP_CUT_SCALED) ? 0.f : g.y);
+                const fp_f2 u = __fadd2_rn(y, c[k]);
+                const fp_f2 uu = __fmul2_rn(u, u);
+                const fp_f2 e = __ffma2_rn(f, uu, q[k]);
+                const fp_f2 v = __fmul2_rn(k ? w.y : w.x, make_float2(fp_ex2(e.x), fp_ex2(e.y)));
+                const fp_f2 K = make_float2((e.x < FP_CUT_SCALED) ? 0.f : v.x, (e.y < FP_CUT_SCALED) ? 0.f : v.y);
                 Y[0][k] = __fadd2_rn(Y[0][k], K);
-                Y[1][k] = __ffma2_rn(K, dy, Y[1][k]);
-                const fp_f2 t = __fmul2_rn(K, yy);
+                Y[1][k] = __ffma2_rn(K, u, Y[1][k]);
+                const fp_f2 t = __fmul2_rn(K, uu);
                 Y[2][k] = __fadd2_rn(Y[2][k], t);
-                Y[3][k] = __ffma2_rn(t, dy, Y[3][k]);
-                Y[4][k] = __ffma2_rn(t, yy, Y[4][k]);
+                Y[3][k] = __ffma2_rn(t, u, Y[3][k]);
+                Y[4][k] = __ffma2_rn(t, uu, Y[4][k]);
             }
-        }
-        // m[i][j] = sum K dx^i dy^j over the strip
-#pragma unroll
-        for (int j = 0; j < 5; ++j) {
-            const float t[4] = {Y[j][0].x, Y[j][0].y, Y[j][1].x, Y[j][1].y};
-            m[0][j] = (t[0] + t[1]) + (t[2] + t[3]);
-            float p[4] = {t[0], t[1], t[2], t[3]};
-#pragma unroll
-            for (int i = 1; i < 5 - j; ++i) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) p[k] *= dx[k];
-                m[i][j] = (p[0] + p[1]) + (p[2] + p[3]);
-            }
+            y = __fadd2_rn(y, ystep);
         }
     }
-    // H = h + |F dx|^2 / 24, h = 1 - tr F / 24
+    // m[i][j] = sum K dx^i u^j over the strip: the sums over its columns k of
+    // k^i Y[j], then shifted by the first column's dx (synthetic division)
+    double m[5][5];
+    const double d = (double)x - (double)xc;
+#pragma unroll
+    for (int j = 4; j >= 0; --j) {
+        const double t0 = Y[j][0].x, t1 = Y[j][0].y, t2 = Y[j][1].x, t3 = Y[j][1].y;
+        double z[5] = {(t0 + t1) + (t2 + t3), t1 + 2.0 * t2 + 3.0 * t3, t1 + 4.0 * t2 + 9.0 * t3,
+                       t1 + 8.0 * t2 + 27.0 * t3, t1 + 16.0 * t2 + 81.0 * t3};
+#pragma unroll
+        for (int i = 0; i < 5 - j; ++i) {
+            m[i][j] = z[0];
+#pragma unroll
+            for (int l = 0; l + 1 < 5 - j - i; ++l) z[l] = d * z[l] + z[l + 1];
+        }
+    }
+    // In ridge coordinates F is diag(al, c), and the pixel axes' metric is
+    // (1, s; s, la): F dx = n (dx, u), |F dx|^2 / 24 = p dx^2 + q dx u + z u^2
+    const double a = J[n_gauss], b = J[2 * n_gauss], c = J[3 * n_gauss], s = ridge.x;
+    const double al = a - s * b - s * (b - s * c), la = 1.0 + s * s;
+    const double n12 = s * c, n21 = s * al, n22 = la * c;
+    const double h = 1.0 - (a + c) * (1.0 / 24.0), p = al * al * (1.0 / 24.0), q = al * n12 * (1.0 / 12.0),
+                 z = c * n22 * (1.0 / 24.0);
+    const double H10 = h * m[1][0] + p * m[3][0] + q * m[2][1] + z * m[1][2];
+    const double H01 = h * m[0][1] + p * m[2][1] + q * m[1][2] + z * m[0][3];
+    const double H20 = h * m[2][0] + p * m[4][0] + q * m[3][1] + z * m[2][2];
+    const double H11 = h * m[1][1] + p * m[3][1] + q * m[2][2] + z * m[1][3];
+    const double H02 = h * m[0][2] + p * m[2][2] + q * m[1][3] + z * m[0][4];
+    const double m0 = m[0][0] * (1.0 / 24.0);
+    S[0] += h * m[0][0] + p * m[2][0] + q * m[1][1] + z * m[0][2];
+    S[1] += H10 - (al * m[1][0] + n12 * m[0][1]) * (1.0 / 12.0);
+    S[2] += H01 - (n21 * m[1][0] + n22 * m[0][1]) * (1.0 / 12.0);
+    S[3] += -0.5 * H20 + (al * m[2][0] + n12 * m[1][1]) * (1.0 / 12.0) - m0;
+    S[4] += -0.5 * H02 + (n21 * m[1][1] + n22 * m[0][2]) * (1.0 / 12.0) - la * m0;
+    S[5] += -H11 + (n21 * m[2][0] + (n22 + al) * m[1][1] + n12 * m[0][2]) * (1.0 / 12.0) - 2.0 * s * m0;
+}
+
+// The image-space partials from a segment's sums in ridge coordinates
+// (dy = u - s dx), with what the FP32 s misses of Fxy / Fyy.
+__device__ __forceinline__ void ridge_to_partials(const double s, const double *__restrict__ J, int64_t n_gauss,
+                                                  double (&S)[6])
+{
     const double a = J[n_gauss], b = J[2 * n_gauss], c = J[3 * n_gauss];
-    const double t = a + c;
-    const double xx = a * a + b * b, xy = b * t, yy = b * b + c * c;      // F^2
-    const double h = 1.0 - t * (1.0 / 24.0);
-    const double p = xx * (1.0 / 24.0), q = xy * (1.0 / 12.0), s = yy * (1.0 / 24.0);
-    const double H10 = h * m[1][0] + p * m[3][0] + q * m[2][1] + s * m[1][2];
-    const double H01 = h * m[0][1] + p * m[2][1] + q * m[1][2] + s * m[0][3];
-    const double H20 = h * m[2][0] + p * m[4][0] + q * m[3][1] + s * m[2][2];
-    const double H11 = h * m[1][1] + p * m[3][1] + q * m[2][2] + s * m[1][3];
-    const double H02 = h * m[0][2] + p * m[2][2] + q * m[1][3] + s * m[0][4];
-    S[0] += h * m[0][0] + p * m[2][0] + q * m[1][1] + s * m[0][2];
-    S[1] += a * H10 + b * H01 - (xx * m[1][0] + xy * m[0][1]) * (1.0 / 12.0);
-    S[2] += b * H10 + c * H01 - (xy * m[1][0] + yy * m[0][1]) * (1.0 / 12.0);
-    S[3] += -0.5 * H20 - m[0][0] * (1.0 / 24.0) + (a * m[2][0] + b * m[1][1]) * (1.0 / 12.0);
-    S[4] += -0.5 * H02 - m[0][0] * (1.0 / 24.0) + (b * m[1][1] + c * m[0][2]) * (1.0 / 12.0);
-    S[5] += -H11 + (b * ((double)m[2][0] + m[0][2]) + t * m[1][1]) * (1.0 / 12.0);
+    const double gx = S[1], gu = S[2];
+    S[1] = (a - s * b) * gx + b * gu;
+    S[2] = (b - s * c) * gx + c * gu;
+    S[4] += s * (s * S[3] - S[5]);
+    S[5] -= 2.0 * s * S[3];
 }
 #endif
 
 struct tile_smem {
-    size_t g, box, pix, wsrc, red, ints, rows, keepw, idx, total;
+    size_t g, ridge, box, pix, wsrc, red, ints, rows, keepw, idx, total;
 };
 
 __host__ __device__ inline tile_smem tile_smem_layout(int tile_pixels, int max_gauss)
@@ -936,6 +1008,7 @@ __host__ __device__ inline tile_smem tile_smem_layout(int tile_pixels, int max_g
     tile_smem L;
     size_t o = 0;
     L.g = o;    o += (size_t)FP_CHUNK * 3 * sizeof(fp_f4);
+    L.ridge = o; o += (size_t)FP_CHUNK * sizeof(fp_f2);
     L.box = o;  o += (size_t)FP_CHUNK * 16;
     L.pix = o;  o += (size_t)tile_pixels * 16;
     L.wsrc = o; o += (size_t)FP_WARPS * MAXSOURCES * NPARAMS * 8;
@@ -953,6 +1026,12 @@ __host__ __device__ inline tile_smem tile_smem_layout(int tile_pixels, int max_g
 // ---------------------------------------------------------------------------
 // P: pixels per thread of the plan's largest tile class (shared memory holds
 // 256 P pixels); each tile runs the forward pass of its own class.
+// 64 registers: four CTAs to an SM.  The compiler then spills 410 bytes in the
+// two larger classes and 226 in the smallest, outside the pixel loops (set-up,
+// the FP64 step of a strip, the segment tree).  At 80 registers and three CTAs
+// it spills 196, and runs the 30-source patch of 32 exposures in 0.92 ms
+// instead of 0.94, the 16-source patch in 93 us instead of 91, 48 field patches
+// in 3.91 ms instead of 3.87.
 template <int P>
 __global__ void __launch_bounds__(FP_THREADS, 4)
 tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc *__restrict__ expos,
@@ -966,7 +1045,7 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
     extern __shared__ __align__(16) unsigned char smem[];
     const tile_smem L = tile_smem_layout(T, max_gauss);
     fp_f4 *s_g = reinterpret_cast<fp_f4 *>(smem + L.g);
-    const staged_gauss sg = {s_g, s_g + FP_CHUNK, s_g + 2 * FP_CHUNK};
+    const staged_gauss sg = {s_g, s_g + FP_CHUNK, s_g + 2 * FP_CHUNK, reinterpret_cast<fp_f2 *>(smem + L.ridge)};
     float4 *s_gbox = reinterpret_cast<float4 *>(smem + L.box);
     float4 *s_pix = reinterpret_cast<float4 *>(smem + L.pix);
     // per-warp source gradients [warp][source][param]: each warp adds its own
@@ -1068,13 +1147,13 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
         tile_grid grid = tile_grid_of(tl, ox, oy, !(flags & (FP_FLAG_FORWARD_ONLY | FP_FLAG_PIXEL_LIST)));
 #endif
         if (tl.tile_pixels == 1024)
-            nzt = forward_tile<4>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, ox, oy, nocull, gc, s_idx, sg, s_gbox, s_pix,
+            nzt = forward_tile<4>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, gjac, n_gauss, ox, oy, nocull, gc, s_idx, sg, s_gbox, s_pix,
                                   s_int, s_red, s_wsrc, s_rows, grid);
         else if (tl.tile_pixels == 512)
-            nzt = forward_tile<2>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, ox, oy, nocull, gc, s_idx, sg, s_gbox, s_pix,
+            nzt = forward_tile<2>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, gjac, n_gauss, ox, oy, nocull, gc, s_idx, sg, s_gbox, s_pix,
                                   s_int, s_red, s_wsrc, s_rows, grid);
         else
-            nzt = forward_tile<1>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, ox, oy, nocull, gc, s_idx, sg, s_gbox, s_pix,
+            nzt = forward_tile<1>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, gjac, n_gauss, ox, oy, nocull, gc, s_idx, sg, s_gbox, s_pix,
                                   s_int, s_red, s_wsrc, s_rows, grid);
         for (int t = tid; t < FP_WARPS * MAXSOURCES * NPARAMS; t += FP_THREADS) s_wsrc[t] = 0.0;
 
@@ -1087,6 +1166,7 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
                 for (int i = tid; i < cn; i += FP_THREADS) {
                     const int64_t gi = ed.gauss_offset + s_idx[c0 + i];
                     stage(sg, i, gfwd, gctr, gi, ox, oy);
+                    if (grid.on) stage_ridge(sg, i, gjac + gi, n_gauss);
                 }
             }
             // the (group of 32 Gaussians) x (unit) plane, split evenly over the
@@ -1144,6 +1224,7 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
                 if (grid.on) {
                     // units run down the rows of one strip, then the next; replica
                     // rep takes rows rep, rep + kr, ...
+                    const fp_f2 ridge = sg.ridge[valid ? gl : 0];
                     int first = 0;
 #pragma unroll 1
                     for (int j = 0; j < 8 && first < q1; ++j) {
@@ -1153,10 +1234,12 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
                         first += n;
                         if (b0 >= b1) continue;
                         const int rend = lo + min(nrow, b1 * kr);
-                        grid_partials(A, fyy, J, n_gauss, reinterpret_cast<const float *>(s_pix) + 4 * j,
+                        grid_partials(A.x, A.y, fyy, ridge, J, n_gauss,
+                                      reinterpret_cast<const float *>(s_pix) + 4 * j,
                                       valid ? lo + b0 * kr + rep : rend, rend, kr, grid.x0 + (float)(4 * j),
                                       grid.y0, S);
                     }
+                    ridge_to_partials(ridge.x, J, n_gauss, S);
                 } else
 #endif
                 {
