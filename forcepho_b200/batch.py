@@ -16,6 +16,8 @@ chi2 and derivatives back to the host, returned per patch in the reference's
 shapes.
 """
 
+import weakref
+
 import numpy as np
 import torch
 
@@ -30,6 +32,28 @@ __all__ = ["BatchedProposer", "render_models"]
 # a source record as raw bytes, for plain copies into the pinned staging buffer
 _RECORD = np.dtype("V%d" % source_struct_dtype.itemsize)
 _ZERO_RECORD = np.zeros(1, dtype=source_struct_dtype).view(_RECORD)[0]
+
+# buffers of proposers that went during a stream capture, where nothing can wait
+_RETIRED = []
+
+
+def _release(done, held):
+    """Let go of a proposer's transfer buffers once the kernels that read or
+    write them are through (``done``: their events).  torch's host allocator
+    knows of its own copies only: it would hand a block that a queued kernel
+    still addresses to the next caller."""
+    if not done:
+        return
+    _RETIRED.append((done, held))
+    if torch.cuda.is_current_stream_capturing():
+        return                          # left to the next proposer that goes
+    while True:
+        try:
+            done, held = _RETIRED.pop()
+        except IndexError:
+            return
+        for event in done.values():
+            event.synchronize()
 
 
 class BatchedProposer:
@@ -84,11 +108,14 @@ class BatchedProposer:
         self._rows = to_device_bytes(rows, dev)
         self._pin_chi2 = torch.zeros(len(rows), dtype=torch.float64).pin_memory()
         self._pin_grad = torch.zeros(max(n_grad, 1), dtype=torch.float32).pin_memory()
-        # completion of the last copy out of the proposal staging buffer and of
-        # the last copy into the result buffers: the host waits on them before
-        # rewriting the one or reading the others
-        self._h2d_done = None
-        self._d2h_done = None
+        # completion of the last copy out of the proposal staging buffer ("h2d")
+        # and of the last copy into the result buffers ("d2h"): the host waits on
+        # them before rewriting the one, reading the others or letting them go
+        self._done = {}
+        self._finalizer = weakref.finalize(self, _release, self._done,
+                                           (self._pin_prop, self._pin_chi2, self._pin_grad, self._counts, self._rows,
+                                            self.plan))
+        self._finalizer.atexit = False
 
     # --- launch parameters ---
     def _autotune(self, tuner, per_class=False):
@@ -141,8 +168,8 @@ class BatchedProposer:
             raise ValueError("%d proposals for %d patches" % (len(proposals), self.n))
         s = stream or torch.cuda.current_stream()
         self.plan.check_current(s)           # a captured graph replays the plan's tables
-        if self._h2d_done is not None:
-            self._h2d_done.synchronize()     # the previous copy may still read the buffer
+        if "h2d" in self._done:
+            self._done["h2d"].synchronize()  # the previous copy may still read the buffer
         slots, lens = self._prop_slots, self._prop_len
         for i in range(self.n):
             if i < len(proposals):
@@ -159,11 +186,16 @@ class BatchedProposer:
             if k < lens[i]:
                 slots[i, k:lens[i]] = _ZERO_RECORD
             lens[i] = k
-        N.check(self.plan.L.fp_upload_proposals(self._pin_prop.data_ptr(), self._counts.data_ptr(), self.n,
-                                                self.plan.proposals.data_ptr(), current_stream_ptr(s)),
-                "fp_upload_proposals")
-        self._h2d_done = torch.cuda.Event()
-        self._h2d_done.record(s)
+        with torch.cuda.device(s.device):    # a launch goes to the current device
+            N.check(self.plan.L.fp_upload_proposals(self._pin_prop.data_ptr(), self._counts.data_ptr(), self.n,
+                                                    self.plan.proposals.data_ptr(), current_stream_ptr(s)),
+                    "fp_upload_proposals")
+        self._mark("h2d", s)
+
+    def _mark(self, name, stream):
+        event = torch.cuda.Event()
+        event.record(stream)
+        self._done[name] = event
 
     def run(self, stream=None):
         """Queue one evaluation of the device proposals (graph replay when captured)."""
@@ -193,18 +225,18 @@ class BatchedProposer:
         """Queue the copy of the existing (patch, band) rows into pinned host memory."""
         s = stream or torch.cuda.current_stream()
         pl = self.plan
-        N.check(pl.L.fp_fetch_results(pl.chi2.data_ptr(), pl.response.data_ptr(), self._rows.data_ptr(),
-                                      self._pin_chi2.numel(), self._pin_chi2.data_ptr(), self._pin_grad.data_ptr(),
-                                      current_stream_ptr(s)), "fp_fetch_results")
-        self._d2h_done = torch.cuda.Event()
-        self._d2h_done.record(s)
+        with torch.cuda.device(s.device):
+            N.check(pl.L.fp_fetch_results(pl.chi2.data_ptr(), pl.response.data_ptr(), self._rows.data_ptr(),
+                                          self._pin_chi2.numel(), self._pin_chi2.data_ptr(),
+                                          self._pin_grad.data_ptr(), current_stream_ptr(s)), "fp_fetch_results")
+        self._mark("d2h", s)
 
     def results(self):
         """Per patch (chi2[n_bands] f64, dchi2[n_bands, n_sources, 7] f32) from the
         last fetch (waiting for its copies to land): views into one fresh copy
         of the fetched rows, so they stay valid after later calls."""
-        if self._d2h_done is not None:
-            self._d2h_done.synchronize()
+        if "d2h" in self._done:
+            self._done["d2h"].synchronize()
         c = self._pin_chi2.numpy().copy()
         g = self._pin_grad.numpy().copy()
         return [(c[a], g[b].reshape(shape)) for a, b, shape in self._slices]
