@@ -56,27 +56,61 @@ std::mutex g_mu;
 std::vector<ref_plan> g_plans;
 unsigned long long g_clock = 0;
 
-// Page-locked landing place of the read-backs, used under g_mu and kept until
-// fp_evaluate_proposal_release(); grown to the largest patch's index arrays.
-unsigned char *g_pinned = nullptr;
-size_t g_pinned_bytes = 0;
+// Page-locked landing places of the read-backs, one per call under way: a call
+// waits for its stream before it takes g_mu, so that work queued on one stream
+// holds up no other thread's call.  Those not in use are kept for later calls,
+// at most MAX_LANDINGS of them, until fp_evaluate_proposal_release().
+struct landing_place {
+    unsigned char *p = nullptr;
+    size_t bytes = 0;
+};
+constexpr size_t MAX_LANDINGS = 8;
+std::mutex g_landing_mu;
+landing_place g_landings[MAX_LANDINGS];
+size_t g_n_landings = 0;
 
-int pinned(size_t bytes, unsigned char **out)
-{
-    if (bytes > g_pinned_bytes) {
-        if (g_pinned) cudaFreeHost(g_pinned);
-        g_pinned = nullptr;
-        g_pinned_bytes = 0;
-        void *p = nullptr;
-        const size_t n = bytes < 4096 ? 4096 : bytes;
-        if (int rc = fp_check_cuda(cudaHostAlloc(&p, n, cudaHostAllocPortable), "fp_evaluate_proposal: host buffer"))
-            return rc;
-        g_pinned = static_cast<unsigned char *>(p);
-        g_pinned_bytes = n;
+class landing {
+public:
+    landing()
+    {
+        std::lock_guard<std::mutex> lock(g_landing_mu);
+        if (g_n_landings > 0) m = g_landings[--g_n_landings];
     }
-    *out = g_pinned;
-    return FP_OK;
-}
+    ~landing()
+    {
+        if (!m.p) return;
+        {
+            std::lock_guard<std::mutex> lock(g_landing_mu);
+            if (g_n_landings < MAX_LANDINGS) {
+                g_landings[g_n_landings++] = m;
+                return;
+            }
+        }
+        cudaFreeHost(m.p);
+    }
+    landing(const landing &) = delete;
+    landing &operator=(const landing &) = delete;
+
+    // room for `bytes` (none of the call's copies may be under way)
+    int ensure(size_t bytes, unsigned char **out)
+    {
+        if (bytes > m.bytes) {
+            if (m.p) cudaFreeHost(m.p);
+            m = landing_place();
+            void *p = nullptr;
+            const size_t n = bytes < 4096 ? 4096 : bytes;
+            if (int rc = fp_check_cuda(cudaHostAlloc(&p, n, cudaHostAllocPortable), "fp_evaluate_proposal: host buffer"))
+                return rc;
+            m.p = static_cast<unsigned char *>(p);
+            m.bytes = n;
+        }
+        *out = m.p;
+        return FP_OK;
+    }
+
+private:
+    landing_place m;
+};
 constexpr size_t MAX_PLANS = 64;
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -219,15 +253,11 @@ extern "C" int fp_evaluate_proposal(const fp_patch *d_patch, const fp_source *d_
     int dev = 0;
     if (int rc = fp_check_cuda(cudaGetDevice(&dev), "cudaGetDevice")) return rc;
 
-    std::lock_guard<std::mutex> lock(g_mu);
-    ref_plan *hit = nullptr;
-    for (ref_plan &p : g_plans)
-        if (p.device == dev && p.d_patch == d_patch) hit = &p;
-
     // 1. the struct
     const size_t nb = (size_t)n_bands;
+    landing place;
     unsigned char *host = nullptr;
-    if (int rc = pinned(sizeof(fp_patch), &host)) return rc;
+    if (int rc = place.ensure(sizeof(fp_patch), &host)) return rc;
     if (int rc = fp_check_cuda(cudaMemcpyAsync(host, d_patch, sizeof(fp_patch), cudaMemcpyDeviceToHost, st),
                                "fp_evaluate_proposal: read patch struct"))
         return rc;
@@ -238,6 +268,11 @@ extern "C" int fp_evaluate_proposal(const fp_patch *d_patch, const fp_source *d_
         return fp_set_error(FP_ERR_ARGUMENT, "fp_evaluate_proposal: n_sources=%d but the patch has %d", n_sources,
                             hp.n_sources);
 
+    std::lock_guard<std::mutex> lock(g_mu);
+    ref_plan *hit = nullptr;
+    for (ref_plan &p : g_plans)
+        if (p.device == dev && p.d_patch == d_patch) hit = &p;
+
     // 2. the index arrays (the exposure arrays sized from band_N, known from
     // the cached plan when the layout has not changed)
     ref_plan cur;
@@ -246,7 +281,7 @@ extern "C" int fp_evaluate_proposal(const fp_patch *d_patch, const fp_source *d_
     const size_t n_exp_guess = (hit && same_layout(hit->key, hp)) ? hit->exposure_start.size() : 0;
     const size_t o_bn = align256(nb * sizeof(int16_t)), o_psf = 2 * o_bn, o_es = align256(o_psf + nb * sizeof(int32_t));
     const size_t o_en = align256(o_es + n_exp_guess * sizeof(int32_t));
-    if (int rc = pinned(o_en + n_exp_guess * sizeof(int32_t), &host)) return rc;
+    if (int rc = place.ensure(o_en + n_exp_guess * sizeof(int32_t), &host)) return rc;
     const auto ask = [&](size_t o, const void *src, size_t n, const char *what) {
         if (n == 0) return (int)FP_OK;
         if (!src) return fp_set_error(FP_ERR_ARGUMENT, "fp_evaluate_proposal: patch without %s", what);
@@ -318,8 +353,7 @@ extern "C" int fp_evaluate_proposal_release(void)
     std::lock_guard<std::mutex> lock(g_mu);
     for (ref_plan &p : g_plans) free_plan(p);
     g_plans.clear();
-    if (g_pinned) cudaFreeHost(g_pinned);
-    g_pinned = nullptr;
-    g_pinned_bytes = 0;
+    std::lock_guard<std::mutex> landing_lock(g_landing_mu);
+    while (g_n_landings > 0) cudaFreeHost(g_landings[--g_n_landings].p);
     return FP_OK;
 }

@@ -207,7 +207,9 @@ FP_API int fp_evaluate_proposal_f64(const fp_patch *d_patch, const fp_source *d_
  * about 208 B per image Gaussian plus 40 B per pixel tile) are device memory
  * owned by the library, at most 64 of them (least recently used first out),
  * until fp_evaluate_proposal_release.  Calls on one patch must not overlap on
- * the GPU: they share its plan's workspace.  n_sources must equal the struct's
+ * the GPU: they share its plan's workspace.  Calls on other patches may come
+ * from other threads, on streams of their own: a call waits for the work
+ * queued on its stream before it takes the lock on the plans.  n_sources must equal the struct's
  * n_sources (FP_ERR_ARGUMENT otherwise). */
 FP_API int fp_evaluate_proposal(const fp_patch *d_patch, const fp_source *d_sources, int n_sources,
                                 int n_bands, double *d_chi2, fp_response *d_response, void *stream);
