@@ -39,6 +39,12 @@ from .kernel_limits import NPARAMS
 __all__ = ["BatchChi2", "PatchChi2"]
 
 
+def _in_memory(t):
+    """``t`` with its values in memory: kernels read addresses, which show neither
+    the pending sign of a negated view nor anything of a zero tensor."""
+    return t.clone() if t._is_zerotensor() else t.resolve_neg()
+
+
 class _Chi2Fn(torch.autograd.Function):
 
     @staticmethod
@@ -106,7 +112,7 @@ class BatchChi2(torch.nn.Module):
         (chi2 rows, their derivatives), as ``fp_fetch_results`` lays them out."""
         if theta.shape != (self.n_params,):
             raise ValueError("theta has shape %s, expected (%d,)" % (tuple(theta.shape), self.n_params))
-        th = theta.to(device=self.device, dtype=torch.float64).contiguous()
+        th = _in_memory(theta.to(device=self.device, dtype=torch.float64)).contiguous()
         s = current_stream_ptr()
         pl = self.plan
         N.check(self.L.fp_hmc_prepare(self.d_hp.data_ptr(), self.n, th.data_ptr(), None, None,
@@ -124,9 +130,14 @@ class BatchChi2(torch.nn.Module):
         """theta gradient of sum_rows grad_chi2[row] * chi2[row], in one launch
         of 2 us (15 torch kernels over every slot took 40 us of the device and
         bound small patches by their launches)."""
-        if torch.is_grad_enabled() and grad_chi2.requires_grad:
+        if grads.device != self.device or grads.shape != (max(self._n_grads, 1),):
+            # only a saved-tensor hook can have changed them
+            raise RuntimeError("the saved derivatives came back as %s on %s, expected [%d] on %s"
+                               % (list(grads.shape), grads.device, max(self._n_grads, 1), self.device))
+        if (torch.is_grad_enabled() and grad_chi2.requires_grad) or grads.dtype != torch.float32:
             return self._vjp_differentiable(grad_chi2, grads)
-        g = grad_chi2.detach().to(torch.float64)
+        g = _in_memory(grad_chi2.detach().to(torch.float64))
+        grads = _in_memory(grads).contiguous()
         out = torch.empty(self.n_params, dtype=torch.float64, device=self.device)
         N.check(self.L.fp_chi2_vjp(self.d_hp.data_ptr(), self.n, self._rows.data_ptr(), self._first_row.data_ptr(),
                                    g.data_ptr(), g.stride(0), grads.data_ptr(), out.data_ptr(),
@@ -135,7 +146,8 @@ class BatchChi2(torch.nn.Module):
 
     def _vjp_differentiable(self, grad_chi2, grads):
         """The same product in torch operations, for a backward pass that is
-        itself differentiated by grad_chi2 (create_graph)."""
+        itself differentiated by grad_chi2 (create_graph), and for derivatives
+        that a saved-tensor hook returned in another type."""
         i64 = dict(dtype=torch.int64, device=self.device)
         out = torch.zeros(self.n_params, dtype=torch.float64, device=self.device)
         for p, sl, rows in zip(self.patches, self.slices, self.band_slices):
