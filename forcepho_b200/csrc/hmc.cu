@@ -96,9 +96,9 @@ constexpr int PREPARE_WARPS = 2;
 
 template <int DEG>
 __global__ void __launch_bounds__(32 * PREPARE_WARPS)
-prepare_kernel(const fp_hmc_patch *__restrict__ hp, const double *__restrict__ z, const double *__restrict__ lower,
-               const double *__restrict__ upper, fp_spline_table tab, fp_source *__restrict__ props,
-               double *__restrict__ theta, double *__restrict__ jac)
+prepare_kernel(const fp_hmc_patch *__restrict__ hp, const double *z, const double *__restrict__ lower,
+               const double *__restrict__ upper, fp_spline_table tab, fp_source *__restrict__ props, double *theta,
+               double *__restrict__ jac)
 {
     const int p = blockIdx.x, lane = threadIdx.x & 31;
     const int s = blockIdx.y * PREPARE_WARPS + (threadIdx.x >> 5);
@@ -119,8 +119,13 @@ prepare_kernel(const fp_hmc_patch *__restrict__ hp, const double *__restrict__ z
         }
         return q;
     };
+    // sersic for the lower half of the warp, rhalf for the upper: read ahead of
+    // the writes, as theta may lie where z does
+    const int half = lane >> 4;
+    double J;
+    const double shape = value(nb + 4 + half, &J);
+    __syncwarp();
     for (int k = lane; k < nper; k += 32) {
-        double J;
         const double q = value(k, &J);
         theta[j0 + k] = q;
         jac[j0 + k] = J;
@@ -133,12 +138,11 @@ prepare_kernel(const fp_hmc_patch *__restrict__ hp, const double *__restrict__ z
     // spline: the lower half of the warp forms the basis in sersic, the upper
     // half in rhalf.  x is clamped to the knots' range first, as FITPACK's
     // bispev/parder do (so does scipy).
-    const int half = lane >> 4;
     const int ncx = tab.nx - tab.kx - 1, ncy = tab.ny - tab.ky - 1;
     const double *t = half ? tab.ty : tab.tx;
     const int n = half ? ncy : ncx, k = half ? tab.ky : tab.kx;
-    double J, N[MAXDEG + 1], dN[MAXDEG + 1];
-    const double x = fmin(fmax(value(nb + 4 + half, &J), t[k]), t[n]);
+    double N[MAXDEG + 1], dN[MAXDEG + 1];
+    const double x = fmin(fmax(shape, t[k]), t[n]);
     const int l = knot_span(t, n, k, x, half ? 0xffff0000u : 0x0000ffffu, lane & 15, 16);
     bspline_basis<DEG>(t, l, k, x, N, dN);
     const int ix = __shfl_sync(0xffffffffu, l, 0) - tab.kx, iy = __shfl_sync(0xffffffffu, l, 16) - tab.ky;
