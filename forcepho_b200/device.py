@@ -321,10 +321,6 @@ class Plan:
         if self._data_stamps() != self._packed:
             self.pack(stream)
 
-    def refresh_patch_pointers(self):
-        ptrs = torch.tensor([p.device_patch_ptr for p in self.patches], dtype=torch.int64)
-        self.d_patches.copy_(ptrs)
-
     @property
     def n_pairs(self):
         return int(self.sizes.n_pairs)
