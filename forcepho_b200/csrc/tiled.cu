@@ -456,7 +456,8 @@ __device__ __forceinline__ int forward_tile(const fp_tile &tl, const fp_exposure
                                             const int32_t *__restrict__ perm, const float4 *__restrict__ pix,
                                             const float4 *__restrict__ gfwd, const float4 *__restrict__ gbox,
                                             const float2 *__restrict__ gctr, const double *__restrict__ gjac,
-                                            const int64_t n_gauss, const float ox, const float oy, const bool nocull, const int gc, const uint16_t *s_idx,
+                                            const int64_t n_gauss, const float ox, const float oy, const bool nocull,
+                                            const int gc, const uint16_t *s_idx,
                                             const staged_gauss &sg, float4 *s_gbox, float4 *s_pix, int *s_int,
                                             double *s_red, double *s_m, unsigned *s_rows, tile_grid &grid)
 {
@@ -882,16 +883,17 @@ __device__ __forceinline__ void partials_to_grad(const double *__restrict__ J, i
 // one per row of 4 pixels.  Four columns are what 64 registers hold (10 sums
 // each pair).
 // Tile kernel on 48 field patches (2.9e9 evaluated pairs): 6.19 ms with the
-// list, 3.77 ms with FP32 sums of plain dy^j, 3.86 ms here; on a 30-source
-// patch of 32 exposures of 256x256 px, 1.64, 0.92 and 0.94 ms; on a 16-source
-// patch of 10 exposures of 150x150 px (256-pixel tiles), 120, 88 and 91 us.
-// The FP64 column sums are 1.5 % of the field patches' time.
+// list, 3.77 ms with FP32 sums of plain dy^j, 3.82 ms here; on a 30-source
+// patch of 32 exposures of 256x256 px, 1.64, 0.92 and 0.93 ms; on a 16-source
+// patch of 10 exposures of 150x150 px (256-pixel tiles), 120, 88 and 90 us.
+// The FP64 column sums are about 1 % of the field patches' time, the whole step
+// at a strip's end 7 %; with F read from the tables at each strip, 8 %.
 //
 // Precision.  Sums of plain dy^j would cancel in E, H and F wherever the
 // Gaussian is thin and oblique; dx and u are the axes in which E has no mixed
 // term.  Any s will do as long as the same one is used throughout: the FP32
-// quotient is, and what it misses of Fxy / Fyy enters the FP64 step.  A column's
-// ridge is held relative to the integer row nearest the strip's, so that its
+// quotient is, and what it misses of Fxy / Fyy enters once per segment.  A
+// column's ridge is held relative to the integer row nearest the strip's, so that its
 // rounding is that of a few pixels, not of the tile's extent.  A column's FP32
 // sum runs over at most 32 pixels, as the list's do, and is FP64 from there on.
 // Largest error of a gradient column against 64 bits on three faint sources
@@ -907,7 +909,6 @@ __device__ __forceinline__ void partials_to_grad(const double *__restrict__ J, i
 // (dx, u) and by the coefficients of (dx^2, u^2, 2 dx u), all but the first as
 // ridge_to_partials takes them.  ridge: the staged pair; fyy: c Fyy.
 __device__ __forceinline__ void grid_partials(const float xc, const float yc, const float fyy, const fp_f2 ridge,
-                                              const double *__restrict__ J, int64_t n_gauss,
                                               const float *__restrict__ s_w, int r, int rend, int step, float x,
                                               float y0, double (&S)[6])
 {
@@ -948,15 +949,15 @@ __device__ __forceinline__ void grid_partials(const float xc, const float yc, co
             y = __fadd2_rn(y, ystep);
         }
     }
-    // m[i][j] = sum K dx^i u^j over the strip: the sums over its columns k of
-    // k^i Y[j], then shifted by the first column's dx (synthetic division)
+    // m[i][j] = sum K dx^i u^j over the strip: the sums of k^i Y[j] over its
+    // columns k = -1 .. 2, then shifted by column 0's dx (synthetic division)
     double m[5][5];
-    const double d = (double)x - (double)xc;
+    const double d = (double)(x + 1.f) - (double)xc;
 #pragma unroll
     for (int j = 4; j >= 0; --j) {
         const double t0 = Y[j][0].x, t1 = Y[j][0].y, t2 = Y[j][1].x, t3 = Y[j][1].y;
-        double z[5] = {(t0 + t1) + (t2 + t3), t1 + 2.0 * t2 + 3.0 * t3, t1 + 4.0 * t2 + 9.0 * t3,
-                       t1 + 8.0 * t2 + 27.0 * t3, t1 + 16.0 * t2 + 81.0 * t3};
+        const double even = t2 + t0, odd = t2 - t0;
+        double z[5] = {(even + t1) + t3, odd + 2.0 * t3, even + 4.0 * t3, odd + 8.0 * t3, even + 16.0 * t3};
 #pragma unroll
         for (int i = 0; i < 5 - j; ++i) {
             m[i][j] = z[0];
@@ -964,13 +965,14 @@ __device__ __forceinline__ void grid_partials(const float xc, const float yc, co
             for (int l = 0; l + 1 < 5 - j - i; ++l) z[l] = d * z[l] + z[l + 1];
         }
     }
-    // In ridge coordinates F is diag(al, c), and the pixel axes' metric is
-    // (1, s; s, la): F dx = n (dx, u), |F dx|^2 / 24 = p dx^2 + q dx u + z u^2
-    const double a = J[n_gauss], b = J[2 * n_gauss], c = J[3 * n_gauss], s = ridge.x;
-    const double al = a - s * b - s * (b - s * c), la = 1.0 + s * s;
-    const double n12 = s * c, n21 = s * al, n22 = la * c;
-    const double h = 1.0 - (a + c) * (1.0 / 24.0), p = al * al * (1.0 / 24.0), q = al * n12 * (1.0 / 12.0),
-                 z = c * n22 * (1.0 / 24.0);
+    // In ridge coordinates F is diag(al, c), as the exponent has it, and the
+    // pixel axes' metric is (1, s; s, la): F dx = n (dx, u), |F dx|^2 / 24 =
+    // p dx^2 + q dx u + z u^2.  al, c and n in twelfths where they are needed so.
+    const double s = ridge.x, la = 1.0 + s * s;
+    const double al = ridge.y * (1.0 / FP_EXP2_SCALE), c = fyy * (1.0 / FP_EXP2_SCALE);
+    const double al12 = al * (1.0 / 12.0), c12 = c * (1.0 / 12.0);
+    const double n12 = s * c12, n21 = s * al12, n22 = la * c12;
+    const double h = 1.0 - 0.5 * (al12 + n22), p = 0.5 * al * al12, q = al * n12, z = 0.5 * c * n22;
     const double H10 = h * m[1][0] + p * m[3][0] + q * m[2][1] + z * m[1][2];
     const double H01 = h * m[0][1] + p * m[2][1] + q * m[1][2] + z * m[0][3];
     const double H20 = h * m[2][0] + p * m[4][0] + q * m[3][1] + z * m[2][2];
@@ -978,11 +980,11 @@ __device__ __forceinline__ void grid_partials(const float xc, const float yc, co
     const double H02 = h * m[0][2] + p * m[2][2] + q * m[1][3] + z * m[0][4];
     const double m0 = m[0][0] * (1.0 / 24.0);
     S[0] += h * m[0][0] + p * m[2][0] + q * m[1][1] + z * m[0][2];
-    S[1] += H10 - (al * m[1][0] + n12 * m[0][1]) * (1.0 / 12.0);
-    S[2] += H01 - (n21 * m[1][0] + n22 * m[0][1]) * (1.0 / 12.0);
-    S[3] += -0.5 * H20 + (al * m[2][0] + n12 * m[1][1]) * (1.0 / 12.0) - m0;
-    S[4] += -0.5 * H02 + (n21 * m[1][1] + n22 * m[0][2]) * (1.0 / 12.0) - la * m0;
-    S[5] += -H11 + (n21 * m[2][0] + (n22 + al) * m[1][1] + n12 * m[0][2]) * (1.0 / 12.0) - 2.0 * s * m0;
+    S[1] += H10 - al12 * m[1][0] - n12 * m[0][1];
+    S[2] += H01 - n21 * m[1][0] - n22 * m[0][1];
+    S[3] += -0.5 * H20 + al12 * m[2][0] + n12 * m[1][1] - m0;
+    S[4] += -0.5 * H02 + n21 * m[1][1] + n22 * m[0][2] - la * m0;
+    S[5] += -H11 + n21 * m[2][0] + (n22 + al12) * m[1][1] + n12 * m[0][2] - 2.0 * s * m0;
 }
 
 // The image-space partials from a segment's sums in ridge coordinates
@@ -1026,12 +1028,11 @@ __host__ __device__ inline tile_smem tile_smem_layout(int tile_pixels, int max_g
 // ---------------------------------------------------------------------------
 // P: pixels per thread of the plan's largest tile class (shared memory holds
 // 256 P pixels); each tile runs the forward pass of its own class.
-// 64 registers: four CTAs to an SM.  The compiler then spills 410 bytes in the
-// two larger classes and 226 in the smallest, outside the pixel loops (set-up,
-// the FP64 step of a strip, the segment tree).  At 80 registers and three CTAs
-// it spills 196, and runs the 30-source patch of 32 exposures in 0.92 ms
-// instead of 0.94, the 16-source patch in 93 us instead of 91, 48 field patches
-// in 3.91 ms instead of 3.87.
+// 64 registers: four CTAs to an SM.  The compiler then spills 434 bytes in the
+// two larger classes and 250 in the smallest.  At 80 registers and three CTAs
+// it spills 196 and 108, and runs the 30-source patch of 32 exposures in 0.91 ms
+// instead of 0.93, the 16-source patch in 92 us instead of 90, 48 field patches
+// in 3.86 ms instead of 3.82.
 template <int P>
 __global__ void __launch_bounds__(FP_THREADS, 4)
 tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc *__restrict__ expos,
@@ -1147,14 +1148,14 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
         tile_grid grid = tile_grid_of(tl, ox, oy, !(flags & (FP_FLAG_FORWARD_ONLY | FP_FLAG_PIXEL_LIST)));
 #endif
         if (tl.tile_pixels == 1024)
-            nzt = forward_tile<4>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, gjac, n_gauss, ox, oy, nocull, gc, s_idx, sg, s_gbox, s_pix,
-                                  s_int, s_red, s_wsrc, s_rows, grid);
+            nzt = forward_tile<4>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, gjac, n_gauss, ox, oy, nocull, gc, s_idx, sg,
+                                  s_gbox, s_pix, s_int, s_red, s_wsrc, s_rows, grid);
         else if (tl.tile_pixels == 512)
-            nzt = forward_tile<2>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, gjac, n_gauss, ox, oy, nocull, gc, s_idx, sg, s_gbox, s_pix,
-                                  s_int, s_red, s_wsrc, s_rows, grid);
+            nzt = forward_tile<2>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, gjac, n_gauss, ox, oy, nocull, gc, s_idx, sg,
+                                  s_gbox, s_pix, s_int, s_red, s_wsrc, s_rows, grid);
         else
-            nzt = forward_tile<1>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, gjac, n_gauss, ox, oy, nocull, gc, s_idx, sg, s_gbox, s_pix,
-                                  s_int, s_red, s_wsrc, s_rows, grid);
+            nzt = forward_tile<1>(tl, ed, pt, perm, pix, gfwd, gbox, gctr, gjac, n_gauss, ox, oy, nocull, gc, s_idx, sg,
+                                  s_gbox, s_pix, s_int, s_red, s_wsrc, s_rows, grid);
         for (int t = tid; t < FP_WARPS * MAXSOURCES * NPARAMS; t += FP_THREADS) s_wsrc[t] = 0.0;
 
         FP_PHASE_MARK(ph2);
@@ -1234,8 +1235,7 @@ tile_kernel(const fp_patch *const *__restrict__ patches, const fp_exposure_desc 
                         first += n;
                         if (b0 >= b1) continue;
                         const int rend = lo + min(nrow, b1 * kr);
-                        grid_partials(A.x, A.y, fyy, ridge, J, n_gauss,
-                                      reinterpret_cast<const float *>(s_pix) + 4 * j,
+                        grid_partials(A.x, A.y, fyy, ridge, reinterpret_cast<const float *>(s_pix) + 4 * j,
                                       valid ? lo + b0 * kr + rep : rend, rend, kr, grid.x0 + (float)(4 * j),
                                       grid.y0, S);
                     }
