@@ -42,7 +42,7 @@ sys.path.insert(0, ROOT)
 METRIC = ("lnlike+grad evals/s and pixel-Gaussian evals/s (batched vs plain, 1 B200, chi2 relerr<=1e-6)")
 UNIT = "pixel-Gaussian evals/s"
 # FP32 flops (FMA = 2) of one forward + adjoint pair evaluation in the direct
-# form (12 moments per pair); the tile kernel does about 33 (power sums down columns)
+# form (12 moments per pair); the tile kernel does about 33 (power sums along ridges)
 FLOPS_PER_PAIR = 84
 EX2_PER_PAIR = 2
 # raw chi2 errors of a band are measured against max(|chi2|, RAW_FLOOR * the
@@ -54,10 +54,10 @@ PARAM_NAMES = ["flux", "ra", "dec", "q", "pa", "sersic", "rhalf"]
 # DRAM bytes (read + write) of one tile_kernel launch, measured by ncu
 # (dram__bytes_read.sum + dram__bytes_write.sum, one pass, the first timed
 # launch of "bench.py --steps 2 --warmup 3 --no-cpu --no-autotune --tile-pixels
-# 1024 --plain-steps 1", NVTX range bench_timed): 6.139 GB read + 0.253 GB
+# 1024 --plain-steps 1", NVTX range bench_timed): 6.313 GB read + 0.258 GB
 # written.  Keyed by (workload, patches, tile pixels) of a one-size plan;
 # other configurations report null.
-TILE_TRAFFIC = {("batched", 512, 1024): 6.139146752e9 + 253.1904e6}
+TILE_TRAFFIC = {("batched", 512, 1024): 6.312696576e9 + 258.36288e6}
 
 
 def hbm_fraction(traffic_bytes, algorithmic_gbs, kernel_ms):
