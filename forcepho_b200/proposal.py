@@ -125,23 +125,27 @@ class B200Proposer(ProposerBase):
         self._pinned_prop.numpy()[:prop.nbytes] = prop.view(np.uint8)     # n_sources records
         stream = torch.cuda.current_stream()
         lp = plan.launch(ctas_per_sm=self.ctas_per_sm, flags=self.flags)
-        if self.use_graph:
-            gkey = (self._plan_key, self.ctas_per_sm, self.flags)
-            if self._graph is None or self._graph_key != gkey:
-                self._capture(plan, lp, stream)
-                self._graph_key = gkey
-            plan.check_current(stream)
-            self._graph.replay()
-        else:
-            self._queue(plan, lp)
-        if patch.return_residual:
-            # outside the graph: a data/residual swap changes its address
-            res = patch.device_ptrs["residual"]
-            nbytes = int(np.prod(res.shape)) * res.dtype.itemsize
-            if self._pinned_res is None or self._pinned_res.numel() < nbytes:
-                self._pinned_res = torch.empty(max(nbytes, 1), dtype=torch.uint8).pin_memory()
-            self._pinned_res[:nbytes].copy_(res.tensor[:nbytes], non_blocking=True)
-        stream.synchronize()
+        try:
+            if self.use_graph:
+                gkey = (self._plan_key, self.ctas_per_sm, self.flags)
+                if self._graph is None or self._graph_key != gkey:
+                    self._capture(plan, lp, stream)
+                    self._graph_key = gkey
+                plan.check_current(stream)
+                self._graph.replay()
+            else:
+                self._queue(plan, lp)
+            if patch.return_residual:
+                # outside the graph: a data/residual swap changes its address
+                res = patch.device_ptrs["residual"]
+                nbytes = int(np.prod(res.shape)) * res.dtype.itemsize
+                if self._pinned_res is None or self._pinned_res.numel() < nbytes:
+                    self._pinned_res = torch.empty(max(nbytes, 1), dtype=torch.uint8).pin_memory()
+                self._pinned_res[:nbytes].copy_(res.tensor[:nbytes], non_blocking=True)
+        finally:
+            # also after an error: the reduction writes the pinned buffers
+            # directly, which torch's host allocator does not know of
+            stream.synchronize()
         chi_out = self._pinned_chi2.numpy()[0, :n_bands].copy()
         chi_derivs = response_view(self._pinned_resp.numpy()[0], n_bands, n_sources).copy()
         if patch.return_residual:

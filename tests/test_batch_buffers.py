@@ -147,3 +147,31 @@ def test_dropping_a_proposer_with_queued_work():
     assert all(bool((t == 7).all()) for t in new)
     again = batch.BatchedProposer([p]).evaluate_proposals(prop)
     np.testing.assert_array_equal(again[0][1], want[0][1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("use_graph", [True, False])
+def test_a_single_call_that_fails_half_way_waits_for_its_kernels(use_graph, monkeypatch):
+    """The reduction writes the proposer's pinned buffers: none of it may be queued once the call is over."""
+    import torch
+    from forcepho_b200 import synthetic as S
+    from forcepho_b200.proposal import B200Proposer
+    p = S.config_multiband(seed=13, n_sources=3, n_bands=2, exp_per_band=1, size=40)
+    p.return_residual = True
+    p.send_to_device()
+    proposer, prop = B200Proposer(use_graph=use_graph), p.scene.get_proposal().copy()
+    want = proposer.evaluate_proposal(prop, patch=p, unpack=False)
+
+    def fails(*args, **kwargs):
+        raise MemoryError("no page-locked memory")
+
+    proposer._pinned_res = None                     # its buffer is made after the launches
+    with monkeypatch.context() as m:
+        m.setattr(torch.Tensor, "pin_memory", fails)
+        torch.cuda._sleep(100_000_000)              # some 50 ms
+        with pytest.raises(MemoryError):
+            proposer.evaluate_proposal(prop, patch=p)
+        assert torch.cuda.current_stream().query()
+    got = proposer.evaluate_proposal(prop, patch=p, unpack=False)
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)
